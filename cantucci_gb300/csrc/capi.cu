@@ -39,6 +39,17 @@ int sm_count() {
     return cache[dev];
 }
 
+// The largest f32 whose (correctly rounded, monotone) square root does not
+// exceed the bailout: |z| > bailout is |z|^2 > this.  NaN for a bailout
+// outside (0, 16], the range p8_de's operations are bounded for.
+static float p8_m2_max(float bailout) {
+    if (!(bailout > 0.0f && bailout <= 16.0f)) return NAN;
+    float t = bailout * bailout;
+    while (sqrtf(t) > bailout) t = nextafterf(t, 0.0f);
+    while (sqrtf(nextafterf(t, INFINITY)) <= bailout) t = nextafterf(t, INFINITY);
+    return t;
+}
+
 // R = Rz(c) Ry(b) Rx(a), row-major, computed in double and rounded to f32.
 __host__ ShapeDev make_shape_dev(const cg_shape& s) {
     ShapeDev d;
@@ -58,6 +69,7 @@ __host__ ShapeDev make_shape_dev(const cg_shape& s) {
     for (int i = 0; i < 3; ++i) d.center[i] = s.center[i];
     d.radius = s.radius;
     d.rotated = s.rot[0] != 0.0f || s.rot[1] != 0.0f || s.rot[2] != 0.0f;
+    d.p8_m2_max = s.max_iters >= 1 ? p8_m2_max(s.bailout) : NAN;
     return d;
 }
 
