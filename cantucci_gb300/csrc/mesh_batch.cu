@@ -665,7 +665,12 @@ cg_status cg_batch_mesh(cg_batch* b, const cg_shape* shape, cg_vertex* vertices,
     if (an) CG_TRY((launch_batch_place<MODE, true>(b, s, vertices, vertex_cap, st))); \
     else CG_TRY((launch_batch_place<MODE, false>(b, s, vertices, vertex_cap, st)));
     switch (mode_of(s, b->numerics)) {
-    case MODE_P8: CG_BATCH_PLACE(MODE_P8) break;  // rolled, as k_place
+    case MODE_P8:
+        if (p8_unrolled(s) && !an) {  // as launch_place
+            CG_TRY((launch_batch_place<MODE_P8_IT15, false>(b, s, vertices, vertex_cap, st)));
+            break;
+        }
+        CG_BATCH_PLACE(MODE_P8) break;
     case MODE_INT: CG_BATCH_PLACE(MODE_INT) break;
     case MODE_POLAR: CG_BATCH_PLACE(MODE_POLAR) break;
     case MODE_P8_FAST:
