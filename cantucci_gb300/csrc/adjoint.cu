@@ -43,6 +43,20 @@ __global__ void __launch_bounds__(128) k_de_grad(ShapeDev s, Dm3 dm, const float
     }
 }
 
+// The same over the long tape (max_iters <= ADJ_LONG_MAX).
+__global__ void __launch_bounds__(ADJ_LONG_BLOCK) k_de_grad_long(ShapeDev s, Dm3 dm,
+                                                                 const float* __restrict__ pts,
+                                                                 uint64_t n,
+                                                                 float* __restrict__ out) {
+    extern __shared__ __align__(16) float long_smem[];
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        float o[8];
+        polar_de_grad_long(s, dm.m, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], long_smem, o);
+        store8(out, i, o);
+    }
+}
+
 template <int T, bool FAST>
 __global__ void __launch_bounds__(128) k_de_grad_tangent(ShapeDev s, Dm3 dm,
                                                          const float* __restrict__ pts, uint64_t n,
@@ -87,16 +101,20 @@ __global__ void __launch_bounds__(128) k_de_spatial_grad(ShapeDev s, const float
 // and, per warp, the sum over its points of g[i] * dDE/d(power, euler) into
 // partial[4 w .. 4 w + 3] (added up by k_sum_partials4 in a fixed order, so
 // the result does not depend on scheduling).
+template <bool LONG>
 __global__ void __launch_bounds__(128) k_de_vjp(ShapeDev s, Dm3 dm, const float* __restrict__ pts,
                                                 const float* __restrict__ g, uint64_t n,
                                                 float* __restrict__ gp, float* __restrict__ params) {
     extern __shared__ __align__(16) float4 adj_smem[];
-    const AdjTape tape = adj_tape(adj_smem, s.max_iters, ADJ_CK);
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         float o[8];
-        polar_de_grad<ADJ_CK>(s, dm.m, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], tape, o);
+        const float x = pts[3 * i], y = pts[3 * i + 1], z = pts[3 * i + 2];
+        if constexpr (LONG)
+            polar_de_grad_long(s, dm.m, x, y, z, reinterpret_cast<float*>(adj_smem), o);
+        else
+            polar_de_grad<ADJ_CK>(s, dm.m, x, y, z, adj_tape(adj_smem, s.max_iters, ADJ_CK), o);
         const float gi = g[i];
         if (gp) {
             gp[3 * i] = gi * o[1];
@@ -304,9 +322,16 @@ template <int CK, bool FR>
 static cg_status launch_de_grad(const ShapeDev& sd, const Dm3& dm, uint32_t max_iters,
                                 const float* points, uint64_t n, float* out, cudaStream_t st) {
     unsigned G = 0;
-    size_t smem = 0;
-    CG_TRY(adj_launch_shape(k_de_grad<CK, FR>, max_iters, CK, n, &G, &smem));
-    k_de_grad<CK, FR><<<G, 128, smem, st>>>(sd, dm, points, n, out);
+    if (CK == ADJ_CK && !FR && max_iters <= ADJ_LONG_MAX) {
+        const size_t smem = long_tape_bytes(max_iters, ADJ_LONG_BLOCK);
+        CG_TRY(adj_launch_shape(k_de_grad_long, ADJ_LONG_BLOCK, smem, n, &G));
+        k_de_grad_long<<<G, ADJ_LONG_BLOCK, smem, st>>>(sd, dm, points, n, out);
+        CG_CHECK_LAUNCH("k_de_grad_long");
+        return CG_OK;
+    }
+    const size_t smem = adj_tape_bytes(max_iters, CK, ADJ_BLOCK);
+    CG_TRY(adj_launch_shape(k_de_grad<CK, FR>, ADJ_BLOCK, smem, n, &G));
+    k_de_grad<CK, FR><<<G, ADJ_BLOCK, smem, st>>>(sd, dm, points, n, out);
     CG_CHECK_LAUNCH("k_de_grad");
     return CG_OK;
 }
@@ -403,14 +428,18 @@ cg_status cg_de_backward(const cg_shape* shape, const float* points, const float
     cudaStream_t st = (cudaStream_t)stream;
     if (grad_params) CG_CUDA(cudaMemsetAsync(grad_params, 0, 4 * sizeof(float), st));
     if (!n) return CG_OK;
+    const bool lng = shape->max_iters <= ADJ_LONG_MAX;
+    const unsigned B = lng ? ADJ_LONG_BLOCK : ADJ_BLOCK;
+    const size_t smem = lng ? long_tape_bytes(shape->max_iters, B)
+                            : adj_tape_bytes(shape->max_iters, ADJ_CK, B);
+    auto kernel = lng ? k_de_vjp<true> : k_de_vjp<false>;
     unsigned G = 0;
-    size_t smem = 0;
-    CG_TRY(adj_launch_shape(k_de_vjp, shape->max_iters, ADJ_CK, n, &G, &smem));
-    const uint32_t nwarps = G * 4;
+    CG_TRY(adj_launch_shape(kernel, B, smem, n, &G));
+    const uint32_t nwarps = G * (B / 32);
     float* partial = nullptr;
     if (grad_params) CG_TRY(acquire_partials((size_t)nwarps * 4, st, &partial));
-    k_de_vjp<<<G, 128, smem, st>>>(make_shape_dev(*shape), rotation_derivatives(*shape), points,
-                                   grad_out, n, grad_points, partial);
+    kernel<<<G, B, smem, st>>>(make_shape_dev(*shape), rotation_derivatives(*shape), points,
+                               grad_out, n, grad_points, partial);
     cg_status rs = cuda_status(cudaGetLastError(), "k_de_vjp", __FILE__, __LINE__);
     if (rs == CG_OK && partial) rs = launch_sum_partials4(partial, nwarps, grad_params, st);
     if (partial) {

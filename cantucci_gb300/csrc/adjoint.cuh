@@ -47,28 +47,6 @@ struct StepState {
     float x, y, z, dr;
 };
 
-// One forward step of the polar loop from (z, dr); returns false on escape
-// (r > bailout).  r is always returned.
-__device__ __forceinline__ bool polar_step(const ShapeDev& s, float qx, float qy, float qz,
-                                           StepState& st, float& r) {
-    r = magnitude<Exact>(st.x, st.y, st.z);
-    if (r > s.bailout) return false;
-    const float P = s.power_f;
-    float theta = acosf(__fdiv_rn(st.z, r));
-    float phi = atan2f(st.y, st.x);
-    st.dr = __fadd_rn(__fmul_rn(__fmul_rn(powf(r, __fsub_rn(P, 1.0f)), P), st.dr), 1.0f);
-    const float zr = powf(r, P);
-    theta = __fmul_rn(theta, P);
-    phi = __fmul_rn(phi, P);
-    float sn, cs, sp, cp;
-    sincosf(theta, &sn, &cs);
-    sincosf(phi, &sp, &cp);
-    st.x = __fadd_rn(__fmul_rn(zr, __fmul_rn(sn, cp)), qx);
-    st.y = __fadd_rn(__fmul_rn(zr, __fmul_rn(sp, sn)), qy);
-    st.z = __fadd_rn(__fmul_rn(zr, cs), qz);
-    return true;
-}
-
 // A step's input and the values its forward computation produces.
 struct StepDeriv {
     float x, y, z, dr;       // z_k, dr_k
@@ -78,20 +56,27 @@ struct StepDeriv {
 };
 constexpr int STEP_FIELDS = 13;
 
-// The step from `st` with |z| = r (not an escape), recorded into `d`: the
-// same operations as polar_step, so the iterate is bit-identical.
+// The step from `st` with |z| = r and z / r = c (not an escape), recorded
+// into `d`: the same operations as polar_step, so the iterate is
+// bit-identical.  `last`: the loop ends here and z stays; nothing flows back
+// into the z that is not formed, so the record's angles and r^P are 0.
 __device__ __forceinline__ void polar_step_rec(const ShapeDev& s, float qx, float qy, float qz,
-                                               float r, StepState& st, StepDeriv& d) {
+                                               float r, float c, StepState& st, StepDeriv& d,
+                                               bool last) {
     d.x = st.x;
     d.y = st.y;
     d.z = st.z;
     d.dr = st.dr;
     d.r = r;
     const float P = s.power_f;
-    d.theta = acosf(__fdiv_rn(st.z, r));
-    d.phi = atan2f(st.y, st.x);
     d.t1 = powf(r, __fsub_rn(P, 1.0f));
     st.dr = __fadd_rn(__fmul_rn(__fmul_rn(d.t1, P), st.dr), 1.0f);
+    if (last) {
+        d.theta = d.phi = d.zr = d.sn = d.cs = d.sp = d.cp = 0.0f;
+        return;
+    }
+    d.theta = acosf(c);
+    d.phi = atan2f(st.y, st.x);
     d.zr = powf(r, P);
     sincosf(__fmul_rn(d.theta, P), &d.sn, &d.cs);
     sincosf(__fmul_rn(d.phi, P), &d.sp, &d.cp);
@@ -181,25 +166,40 @@ __device__ __forceinline__ StepDeriv tape_get(const AdjTape& t, uint32_t slot) {
                      b[7 * n], b[8 * n], b[9 * n], b[10 * n], b[11 * n], b[12 * n]};
 }
 
-// Launch shape of a kernel with a per-thread tape: block 128, dynamic shared
-// memory for the tape (opting in above 48 KB), and a grid of the blocks
-// that fit on the GPU at once (the kernels walk their points grid-stride).
+// The long tape: of every step what the backward sweep cannot form again from
+// its neighbours -- dr, r^(P-1), the two angles, r^P and the sines and cosines
+// (z_k follows from step k - 1's record and q by the step's own operations, r
+// from z_k).  The last step the loop allows needs the first two only.  No
+// checkpoints and no recomputed segments, 512 bytes per thread at 15 steps.
+constexpr int LONG_FIELDS = 9;
+constexpr uint32_t ADJ_LONG_MAX = 20;  // the longest loop that takes it
+
+__host__ __device__ constexpr size_t long_tape_bytes(uint32_t max_iters, uint32_t nth) {
+    return ((size_t)LONG_FIELDS * (max_iters - 1) + 2u) * 4u * nth;
+}
+
+constexpr unsigned ADJ_BLOCK = 128;      // threads per block, checkpointed tape
+constexpr unsigned ADJ_LONG_BLOCK = 64;  // long tape
+
+// Launch shape of a kernel with a per-thread tape in dynamic shared memory
+// (opting in above 48 KB): a grid of the blocks that fit on the GPU at once
+// (the kernels walk their points grid-stride).
 template <class Kernel>
-cg_status adj_launch_shape(Kernel kernel, uint32_t max_iters, int ck, uint64_t n,
-                           unsigned* grid, size_t* smem) {
-    *smem = adj_tape_bytes(max_iters, ck, 128);
-    if (*smem > 48 * 1024)
+cg_status adj_launch_shape(Kernel kernel, unsigned block, size_t smem, uint64_t n,
+                           unsigned* grid) {
+    if (smem > 48 * 1024)
         CG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)*smem));
+                                     (int)smem));
     int per_sm = 0;
-    CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, *smem));
-    *grid = grid_for(n, 128, (unsigned)(per_sm > 0 ? per_sm : 1));
+    CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, (int)block, smem));
+    *grid = grid_for(n, block, (unsigned)(per_sm > 0 ? per_sm : 1));
     return CG_OK;
 }
 
 // Backward through one recorded step (the step formulas at the top of this
 // file).  `stale` adds the seed of the returned r when the loop ran out and
-// this is its last step.
+// this is its last step.  Every FMA is written out, so that the sweep rounds
+// alike wherever it is compiled.
 __device__ __forceinline__ void polar_back_step(float P, const StepDeriv& z, bool stale,
                                                 float r_seed, float& zbx, float& zby, float& zbz,
                                                 float& drb, float& qbx, float& qby, float& qbz,
@@ -208,31 +208,54 @@ __device__ __forceinline__ void polar_back_step(float P, const StepDeriv& z, boo
     qby += zby;
     qbz += zbz;
     const float inv_r = rcp_nr(z.r);
-    const float rho2 = z.x * z.x + z.y * z.y;
+    const float rho2 = fmaf(z.x, z.x, z.y * z.y);
     const float lnr = __logf(z.r);
-    const float g_zr = zbx * (z.sn * z.cp) + zby * (z.sn * z.sp) + zbz * z.cs;
-    const float g_th = z.zr * (zbx * (z.cs * z.cp) + zby * (z.cs * z.sp) - zbz * z.sn);
-    const float g_ph = z.zr * z.sn * (zby * z.cp - zbx * z.sp);
-    float rb = g_zr * P * z.t1 + drb * P * z.dr * (P - 1.0f) * z.t1 * inv_r;
+    const float g_zr = fmaf(zbz, z.cs, fmaf(zby, z.sn * z.sp, zbx * (z.sn * z.cp)));
+    const float g_th = z.zr * fmaf(-zbz, z.sn, fmaf(zby, z.cs * z.sp, zbx * (z.cs * z.cp)));
+    const float g_ph = z.zr * z.sn * fmaf(zby, z.cp, -(zbx * z.sp));
+    float rb = fmaf(drb * P * z.dr * (P - 1.0f) * z.t1, inv_r, g_zr * P * z.t1);
     if (stale) rb += r_seed;
-    Pb += g_zr * z.zr * lnr + g_th * z.theta + g_ph * z.phi + drb * z.dr * z.t1 * (1.0f + P * lnr);
+    Pb += fmaf(drb * z.dr * z.t1, fmaf(P, lnr, 1.0f),
+               fmaf(g_ph, z.phi, fmaf(g_zr * z.zr, lnr, g_th * z.theta)));
     drb = drb * P * z.t1;
     const float thb = P * g_th, phb = P * g_ph;
     const float rbr = rb * inv_r;
-    float gx = rbr * z.x, gy = rbr * z.y, gz = rbr * z.z;
+    zbx = __fmul_rn(rbr, z.x);
+    zby = __fmul_rn(rbr, z.y);
+    zbz = __fmul_rn(rbr, z.z);
     if (rho2 > 1e-30f) {
         const float inv_rho = rsqrtf(rho2);
         const float rho = rho2 * inv_rho;
         const float inv_rho2 = inv_rho * inv_rho;
         const float inv_r2 = inv_r * inv_r;
         const float k = thb * z.z * inv_r2 * inv_rho;
-        gx += k * z.x - phb * z.y * inv_rho2;
-        gy += k * z.y + phb * z.x * inv_rho2;
-        gz += -thb * rho * inv_r2;
+        zbx = __fadd_rn(zbx, fmaf(k, z.x, -(phb * z.y * inv_rho2)));
+        zby = __fadd_rn(zby, fmaf(k, z.y, phb * z.x * inv_rho2));
+        zbz = fmaf(-thb * rho, inv_r2, zbz);
     }
-    zbx = gx;
-    zby = gy;
-    zbz = gz;
+}
+
+// out[0..7] from the swept adjoints of z_0 and q: dDE/dp = R q_bar (q = R^T p)
+// and, per angle, q_bar . (dR/d(angle))^T p.
+__device__ __forceinline__ void grad_outputs(const ShapeDev& s, const float* __restrict__ dm,
+                                             float px, float py, float pz, float de, float zbx,
+                                             float zby, float zbz, float qbx, float qby, float qbz,
+                                             float Pb, float* out) {
+    qbx += zbx;  // z_0 = q
+    qby += zby;
+    qbz += zbz;
+    out[0] = x86_nan(de);
+    out[1] = fmaf(s.m[2], qbz, fmaf(s.m[1], qby, s.m[0] * qbx));
+    out[2] = fmaf(s.m[5], qbz, fmaf(s.m[4], qby, s.m[3] * qbx));
+    out[3] = fmaf(s.m[8], qbz, fmaf(s.m[7], qby, s.m[6] * qbx));
+    out[4] = Pb;
+    for (int a = 0; a < 3; ++a) {
+        const float* d = dm + 9 * a;
+        const float dqx = fmaf(d[6], pz, fmaf(d[0], px, d[3] * py));
+        const float dqy = fmaf(d[7], pz, fmaf(d[1], px, d[4] * py));
+        const float dqz = fmaf(d[8], pz, fmaf(d[2], px, d[5] * py));
+        out[5 + a] = fmaf(qbz, dqz, fmaf(qbx, dqx, qby * dqy));
+    }
 }
 
 // DE and its gradient with respect to p, the power and the Euler angles
@@ -257,14 +280,13 @@ __device__ __forceinline__ void polar_de_grad(const ShapeDev& s, const float* __
     bool escaped = false;
     for (uint32_t i = 0; i < N; ++i) {
         if (i % CK == 0) tape_put_ck(tape, i / CK, st);
-        const float ri = magnitude<Exact>(st.x, st.y, st.z);
-        r = ri;
-        if (ri > s.bailout) {
+        float c;
+        if (!polar_radius(s, magnitude2(st.x, st.y, st.z), st.z, r, c)) {
             escaped = true;
             break;
         }
         StepDeriv d;
-        polar_step_rec(s, qx, qy, qz, ri, st, d);
+        polar_step_rec(s, qx, qy, qz, r, c, st, d, i + 1 == N);
         tape_put(tape, i % CK, d);
         ++K;
     }
@@ -295,10 +317,13 @@ __device__ __forceinline__ void polar_de_grad(const ShapeDev& s, const float* __
                 StepState t = tape_get_ck(tape, (uint32_t)j);
                 for (uint32_t k = k0; k < k1; ++k) {
                     StepDeriv d;
-                    if (FASTREC)
+                    if (FASTREC) {
                         polar_step_rec_fast(P, qx, qy, qz, t, d);
-                    else
-                        polar_step_rec(s, qx, qy, qz, magnitude<Exact>(t.x, t.y, t.z), t, d);
+                    } else {
+                        float rk, c;
+                        polar_radius(s, magnitude2(t.x, t.y, t.z), t.z, rk, c);
+                        polar_step_rec(s, qx, qy, qz, rk, c, t, d, false);
+                    }
                     tape_put(tape, k - k0, d);
                 }
             }
@@ -309,24 +334,106 @@ __device__ __forceinline__ void polar_de_grad(const ShapeDev& s, const float* __
             }
         }
     }
-    // z_0 = q.
-    qbx += zbx;
-    qby += zby;
-    qbz += zbz;
-    out[0] = x86_nan(de);
-    // dDE/dp = R q_bar (q = R^T p).
-    out[1] = s.m[0] * qbx + s.m[1] * qby + s.m[2] * qbz;
-    out[2] = s.m[3] * qbx + s.m[4] * qby + s.m[5] * qbz;
-    out[3] = s.m[6] * qbx + s.m[7] * qby + s.m[8] * qbz;
-    out[4] = Pb;
-    for (int a = 0; a < 3; ++a) {
-        const float* d = dm + 9 * a;
-        // dq/d(angle) = (dR/d(angle))^T p
-        const float dqx = d[0] * px + d[3] * py + d[6] * pz;
-        const float dqy = d[1] * px + d[4] * py + d[7] * pz;
-        const float dqz = d[2] * px + d[5] * py + d[8] * pz;
-        out[5 + a] = qbx * dqx + qby * dqy + qbz * dqz;
+    grad_outputs(s, dm, px, py, pz, de, zbx, zby, zbz, qbx, qby, qbz, Pb, out);
+}
+
+// polar_de_grad over the long tape (long_tape_bytes(s.max_iters, blockDim.x)
+// bytes at `tape`): the same operations and the same records, each formed
+// once.
+__device__ __forceinline__ void polar_de_grad_long(const ShapeDev& s, const float* __restrict__ dm,
+                                                   float px, float py, float pz,
+                                                   float* __restrict__ tape, float* out) {
+    float qx, qy, qz;
+    rotate_point(s, px, py, pz, qx, qy, qz);
+    const float P = s.power_f;
+    const uint32_t N = s.max_iters, n = blockDim.x;
+    tape += threadIdx.x;
+    float x = qx, y = qy, z = qz, dr = 1.0f, r = 0.0f;
+    uint32_t K = 0;
+    bool escaped = false;
+    float* b = tape;
+    for (;;) {
+        float c;
+        if (!polar_radius(s, magnitude2(x, y, z), z, r, c)) {
+            escaped = true;
+            break;
+        }
+        const float t1 = powf(r, __fsub_rn(P, 1.0f));
+        b[0] = dr;
+        b[n] = t1;
+        dr = __fadd_rn(__fmul_rn(__fmul_rn(t1, P), dr), 1.0f);
+        if (++K == N) break;
+        const float theta = acosf(c), phi = atan2f(y, x), zr = powf(r, P);
+        float sn, cs, sp, cp;
+        sincosf(__fmul_rn(theta, P), &sn, &cs);
+        sincosf(__fmul_rn(phi, P), &sp, &cp);
+        b[2 * n] = theta;
+        b[3 * n] = phi;
+        b[4 * n] = zr;
+        b[5 * n] = sn;
+        b[6 * n] = cs;
+        b[7 * n] = sp;
+        b[8 * n] = cp;
+        b += LONG_FIELDS * n;
+        x = __fadd_rn(__fmul_rn(zr, __fmul_rn(sn, cp)), qx);
+        y = __fadd_rn(__fmul_rn(zr, __fmul_rn(sp, sn)), qy);
+        z = __fadd_rn(__fmul_rn(zr, cs), qz);
     }
+    const float ln_r = logf(r);
+    const float de = __fdiv_rn(__fmul_rn(0.5f, __fmul_rn(ln_r, r)), dr);
+    float r_seed = 0.5f * (ln_r + 1.0f) / dr;
+    float drb = -de / dr;
+    float zbx = 0.0f, zby = 0.0f, zbz = 0.0f;
+    if (escaped && r > 0.0f) {
+        const float k = r_seed / r;
+        zbx = k * x;
+        zby = k * y;
+        zbz = k * z;
+        r_seed = 0.0f;
+    }
+    float qbx = 0.0f, qby = 0.0f, qbz = 0.0f, Pb = 0.0f;
+    StepDeriv d = {};
+    if (K > 0 && escaped) {  // else the last step's angles and r^P stay 0
+        b = tape + (size_t)(K - 1) * LONG_FIELDS * n;
+        d.zr = b[4 * n];
+        d.sn = b[5 * n];
+        d.cs = b[6 * n];
+        d.sp = b[7 * n];
+        d.cp = b[8 * n];
+    }
+    for (uint32_t k = K; k-- > 0;) {
+        b = tape + (size_t)k * LONG_FIELDS * n;
+        d.dr = b[0];
+        d.t1 = b[n];
+        const bool stale = !escaped && k + 1 == N;
+        d.theta = stale ? 0.0f : b[2 * n];
+        d.phi = stale ? 0.0f : b[3 * n];
+        float zr = 0.0f, sn = 0.0f, cs = 0.0f, sp = 0.0f, cp = 0.0f;
+        if (k > 0) {  // z_k, by the operations that formed it
+            b -= LONG_FIELDS * n;
+            zr = b[4 * n];
+            sn = b[5 * n];
+            cs = b[6 * n];
+            sp = b[7 * n];
+            cp = b[8 * n];
+            d.x = __fadd_rn(__fmul_rn(zr, __fmul_rn(sn, cp)), qx);
+            d.y = __fadd_rn(__fmul_rn(zr, __fmul_rn(sp, sn)), qy);
+            d.z = __fadd_rn(__fmul_rn(zr, cs), qz);
+        } else {
+            d.x = qx;
+            d.y = qy;
+            d.z = qz;
+        }
+        float c;
+        polar_radius(s, magnitude2(d.x, d.y, d.z), d.z, d.r, c);
+        polar_back_step(P, d, stale, r_seed, zbx, zby, zbz, drb, qbx, qby, qbz, Pb);
+        d.zr = zr;
+        d.sn = sn;
+        d.cs = cs;
+        d.sp = sp;
+        d.cp = cp;
+    }
+    grad_outputs(s, dm, px, py, pz, de, zbx, zby, zbz, qbx, qby, qbz, Pb, out);
 }
 
 // Forward (tangent) mode of the same loop: one pass carries the derivative
@@ -362,64 +469,81 @@ __device__ __forceinline__ void polar_de_tangent(const ShapeDev& s, const float*
         tdr[k] = 0.0f;
         tr[k] = 0.0f;
     }
-    for (uint32_t i = 0; i < s.max_iters; ++i) {
+    for (uint32_t i = 0; i < s.max_iters;) {
+        // One test finds |z| inside the bailout and rho, r and their squares
+        // normal: the roots, reciprocals and the quotient z / r then need
+        // none of their own (the same bits either way).
         const float rho2 = zx * zx + zy * zy;
-        r = FAST ? sqrtf(fmaf(zz, zz, rho2)) : magnitude<Exact>(zx, zy, zz);
-        const float inv_r = 1.0f / r;
+        const float m2 = FAST ? fmaf(zz, zz, rho2) : magnitude2(zx, zy, zz);
+        const bool normal = m2 <= s.m2_max && rho2 >= kPolarMinM2;
+        float inv_r, rho, inv_rho, inv_rho2, c;
+        if (normal) {
+            r = sqrt_rn_normal(m2);
+            inv_r = rcp_rn_normal(r);
+            rho = sqrt_rn_normal(rho2);
+            inv_rho = rcp_rn_normal(rho);
+            inv_rho2 = rcp_rn_normal(rho2);
+            c = FAST ? 0.0f : div_rn_normal(zz, r);
+        } else {
+            r = sqrtf(m2);
+            inv_r = 1.0f / r;
+            rho = sqrtf(rho2);
+            const bool off_axis = rho > 1e-30f;
+            inv_rho = off_axis ? 1.0f / rho : 0.0f;
+            inv_rho2 = off_axis ? 1.0f / rho2 : 0.0f;
+            c = FAST ? 0.0f : __fdiv_rn(zz, r);
+        }
 #pragma unroll
         for (int k = 0; k < T; ++k) tr[k] = (zx * tx[k] + zy * ty[k] + zz * tz[k]) * inv_r;
-        if (r > s.bailout) break;
-        const float rho = sqrtf(rho2);
-        float theta, phi, t1, zr, sn, cs, sp, cp;
-        const float dr_old = dr;
+        if (!normal && r > s.bailout) break;
+        const float lr = FAST ? __log2f(r) : 0.0f;
+        const float t1 = FAST ? exp2f((P - 1.0f) * lr) : powf(r, __fsub_rn(P, 1.0f));
+        const float Pt1 = P * t1;
+        const float k_dr = Pt1 * (P - 1.0f) * inv_r * dr;  // d(dr')/dr
+        float lnr = 0.0f;
+        if (T == 4) lnr = FAST ? __logf(r) : logf(r);
+#pragma unroll
+        for (int k = 0; k < T; ++k) {
+            tdr[k] = k_dr * tr[k] + Pt1 * tdr[k];
+            if (T == 4 && k == 3) tdr[k] += t1 * dr * (1.0f + P * lnr);  // the power direction
+        }
+        dr = FAST ? fmaf(t1 * P, dr, 1.0f)
+                  : __fadd_rn(__fmul_rn(__fmul_rn(t1, P), dr), 1.0f);
+        if (++i == s.max_iters) break;  // nobody reads the last z or its tangents
+        float theta, phi, zr, sn, cs, sp, cp;
         if (FAST) {  // polar_step_fast's arithmetic
             theta = atan2_fast(rho, zz);
             phi = atan2_fast(zy, zx);
-            const float lr = __log2f(r);
             zr = exp2f(P * lr);
-            t1 = exp2f((P - 1.0f) * lr);
-            dr = fmaf(t1 * P, dr, 1.0f);
             sincos_fast(theta * P, &sn, &cs);
             sincos_fast(phi * P, &sp, &cp);
         } else {
-            theta = acosf(__fdiv_rn(zz, r));
+            theta = acosf(c);
             phi = atan2f(zy, zx);
-            t1 = powf(r, __fsub_rn(P, 1.0f));
-            dr = __fadd_rn(__fmul_rn(__fmul_rn(t1, P), dr), 1.0f);
             zr = powf(r, P);
             sincosf(__fmul_rn(theta, P), &sn, &cs);
             sincosf(__fmul_rn(phi, P), &sp, &cp);
         }
-        // shared factors of the tangent step
-        const bool off_axis = rho > 1e-30f;
-        const float inv_rho = off_axis ? 1.0f / rho : 0.0f;
-        const float inv_rho2 = off_axis ? 1.0f / rho2 : 0.0f;
+        // shared factors of the tangent step: u and its derivatives, scaled
+        // by zr
         const float inv_r2 = inv_r * inv_r;
-        const float Pt1 = P * t1;
-        const float k_dr = Pt1 * (P - 1.0f) * inv_r * dr_old;  // d(dr')/dr
-        // u and its derivatives, scaled by zr
         const float ux = sn * cp, uy = sp * sn, uz = cs;
         const float ax = zr * cs * cp, ay = zr * sp * cs, az = -zr * sn;  // zr du/dTh
         const float bx = -zr * sn * sp, by = zr * cp * sn;                // zr du/dPh
-        float lnr = 0.0f;
-        if (T == 4) lnr = FAST ? __logf(r) : logf(r);
 #pragma unroll
         for (int k = 0; k < T; ++k) {
             const float th_t = (zz * (zx * tx[k] + zy * ty[k]) * inv_rho - rho * tz[k]) * inv_r2;
             const float ph_t = (zx * ty[k] - zy * tx[k]) * inv_rho2;
             float zr_t = Pt1 * tr[k];
             float Th_t = P * th_t, Ph_t = P * ph_t;
-            float dr_t = k_dr * tr[k] + Pt1 * tdr[k];
             if (T == 4 && k == 3) {  // the power direction
                 zr_t += zr * lnr;
                 Th_t += theta;
                 Ph_t += phi;
-                dr_t += t1 * dr_old * (1.0f + P * lnr);
             }
             tx[k] = zr_t * ux + Th_t * ax + Ph_t * bx + (k == 0 ? 1.0f : 0.0f);
             ty[k] = zr_t * uy + Th_t * ay + Ph_t * by + (k == 1 ? 1.0f : 0.0f);
             tz[k] = zr_t * uz + Th_t * az + (k == 2 ? 1.0f : 0.0f);
-            tdr[k] = dr_t;
         }
         if (FAST) {
             zx = fmaf(zr, sn * cp, qx);

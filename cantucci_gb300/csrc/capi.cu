@@ -41,9 +41,9 @@ int sm_count() {
 
 // The largest f32 whose (correctly rounded, monotone) square root does not
 // exceed the bailout: |z| > bailout is |z|^2 > this.  NaN for a bailout
-// outside (0, 16], the range p8_de's operations are bounded for.
-static float p8_m2_max(float bailout) {
-    if (!(bailout > 0.0f && bailout <= 16.0f)) return NAN;
+// outside (0, 2^20], where the shortened operations' operands are normal.
+static float largest_square(float bailout) {
+    if (!(bailout > 0.0f && bailout <= 0x1p20f)) return NAN;
     float t = bailout * bailout;
     while (sqrtf(t) > bailout) t = nextafterf(t, 0.0f);
     while (sqrtf(nextafterf(t, INFINITY)) <= bailout) t = nextafterf(t, INFINITY);
@@ -69,7 +69,8 @@ __host__ ShapeDev make_shape_dev(const cg_shape& s) {
     for (int i = 0; i < 3; ++i) d.center[i] = s.center[i];
     d.radius = s.radius;
     d.rotated = s.rot[0] != 0.0f || s.rot[1] != 0.0f || s.rot[2] != 0.0f;
-    d.p8_m2_max = s.max_iters >= 1 ? p8_m2_max(s.bailout) : NAN;
+    d.m2_max = largest_square(s.bailout);
+    d.p8_m2_max = s.max_iters >= 1 && s.bailout <= 16.0f ? d.m2_max : NAN;
     return d;
 }
 

@@ -5,6 +5,7 @@
 #include "common.cuh"
 #include "de.cuh"
 #include "kernels.cuh"
+#include "lane_pool.cuh"
 #include "point_io.cuh"
 
 namespace cg {
@@ -21,6 +22,40 @@ __global__ void __launch_bounds__(256) k_de_points(ShapeDev s, const float* __re
         if (load_point_warp(pts, n, base, stage[threadIdx.x >> 5], x, y, z))
             out[base + (threadIdx.x & 31)] = eval<M>(s, x, y, z);
     }
+}
+
+// Large batches: each warp takes its points through a lane pool.
+template <int M>
+struct PointTask {
+    const ShapeDev& s;
+    const float* __restrict__ pts;
+    float* __restrict__ out;
+    DeLoop<M> de;
+    __device__ __forceinline__ void start(uint64_t i) {
+        de.start(s, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]);
+    }
+    __device__ __forceinline__ bool step() { return de.step(s); }
+    __device__ __forceinline__ void finish(uint64_t i) { out[i] = de.value(s); }
+    __device__ __forceinline__ uint32_t steps() const { return de.it; }
+};
+
+// Lanes that wait in a pool: more where a step is short.
+template <int M>
+constexpr int kPointFlush = M == MODE_P8 || M == MODE_P8_FAST ? 12 : 8;
+
+// MU: the mode of the loop for points side by side.
+template <int M, int MU>
+__global__ void __launch_bounds__(128) k_de_points_pool(ShapeDev s, const float* __restrict__ pts,
+                                                        uint64_t n, float* __restrict__ out) {
+    const WarpWalk w = warp_walk();
+    if (w.first >= n) return;
+    if (points_side_by_side(pts, w, n)) {
+        for (uint64_t i = w.first + (threadIdx.x & 31); i < n; i += w.stride)
+            out[i] = eval<MU>(s, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]);
+        return;
+    }
+    PointTask<M> task{s, pts, out, {}};
+    warp_pool(w, n, kPointFlush<M>, s.max_iters, task);
 }
 
 // Corner (x, y, z) of a span grid: p = start + across * (v / res)
@@ -235,9 +270,41 @@ cg_status launch_grid_work(const ShapeDev& s, const GridDev& g, unsigned long lo
 }
 
 
+template <int M, int MU = M>
+static bool launch_points_pool(const ShapeDev& s, const float* pts, uint64_t n, float* out,
+                               cudaStream_t st) {
+    const unsigned G = pool_grid(k_de_points_pool<M, MU>, n);
+    if (G) k_de_points_pool<M, MU><<<G, 128, 0, st>>>(s, pts, n, out);
+    return G != 0;
+}
+
+// True if the batch is large enough for a pool kernel (and was launched).
+static bool launch_points_pool_mode(const ShapeDev& s, const float* pts, uint64_t n, float* out,
+                                    uint32_t numerics, cudaStream_t st) {
+    if (n < (1u << 18) || s.max_iters < 1) return false;
+    switch (mode_of(s, numerics)) {
+    case MODE_SPHERE: return false;
+    case MODE_P8:
+        return p8_unrolled(s) ? launch_points_pool<MODE_P8, MODE_P8_IT15>(s, pts, n, out, st)
+                              : launch_points_pool<MODE_P8>(s, pts, n, out, st);
+    case MODE_INT: return launch_points_pool<MODE_INT>(s, pts, n, out, st);
+    case MODE_POLAR: return launch_points_pool<MODE_POLAR>(s, pts, n, out, st);
+    case MODE_INT_POLY: return launch_points_pool<MODE_INT_POLY>(s, pts, n, out, st);
+    case MODE_POLAR_FAST: return launch_points_pool<MODE_POLAR_FAST>(s, pts, n, out, st);
+    default:
+        return p8_unrolled(s)
+                   ? launch_points_pool<MODE_P8_FAST, MODE_P8_FAST_IT15>(s, pts, n, out, st)
+                   : launch_points_pool<MODE_P8_FAST>(s, pts, n, out, st);
+    }
+}
+
 cg_status launch_de_points(const ShapeDev& s, const float* pts, uint64_t n, float* out,
                            uint32_t numerics, cudaStream_t st) {
     if (n == 0) return CG_OK;
+    if (launch_points_pool_mode(s, pts, n, out, numerics, st)) {
+        CG_CHECK_LAUNCH("k_de_points_pool");
+        return CG_OK;
+    }
     const unsigned B = 256, G = grid_for(n, B, 16);
     switch (mode_of(s, numerics)) {
     case MODE_P8:

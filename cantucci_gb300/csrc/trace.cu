@@ -17,6 +17,7 @@
 #include "adjoint.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
+#include "lane_pool.cuh"
 
 namespace cg {
 
@@ -63,40 +64,6 @@ __global__ void __launch_bounds__(128) k_trace(ShapeDev s, CameraDev c, uint32_t
     }
 }
 
-// The polar estimator one loop iteration at a time (the same operations as
-// polar_de, or polar_de_fast with FAST), so that a lane can start a new
-// estimate while its warp neighbours are still iterating theirs.
-template <bool FAST>
-struct PolarIter {
-    float qx, qy, qz;  // R^T p
-    StepState st;      // z, dr
-    float r;
-    uint32_t it;
-
-    __device__ __forceinline__ void start(const ShapeDev& s, float px, float py, float pz) {
-        rotate_point<FAST>(s, px, py, pz, qx, qy, qz);
-        st = {qx, qy, qz, 1.0f};
-        r = 0.0f;
-        it = 0;
-    }
-    // One iteration; true when the estimate is complete (escape, or the
-    // last iteration ran: r is then the stale |z| of that iteration).
-    __device__ __forceinline__ bool advance(const ShapeDev& s) {
-        float ri;
-        const bool go = FAST ? polar_step_fast(s.power_f, s.bailout, qx, qy, qz, st.x, st.y,
-                                               st.z, st.dr, ri)
-                             : polar_step(s, qx, qy, qz, st, ri);
-        r = ri;
-        if (!go) return true;
-        return ++it >= s.max_iters;
-    }
-    __device__ __forceinline__ float value() const {
-        if (FAST) return x86_nan(__fdividef(0.5f * __logf(r) * r, st.dr));
-        const float ln_r = __fmul_rn(logf(r), r);
-        return x86_nan(__fdiv_rn(__fmul_rn(0.5f, ln_r), st.dr));
-    }
-};
-
 // The same march with a work queue: persistent warps, and a lane whose ray
 // is finished takes the next pixel at once (one atomic per warp and refill),
 // so a warp no longer waits for its longest ray.  For the polar form the
@@ -114,7 +81,7 @@ __global__ void __launch_bounds__(128) k_trace_queue(ShapeDev s, CameraDev c, ui
     bool done = false;
     float d[3] = {0.0f, 0.0f, 0.0f}, t = 0.0f;
     constexpr bool kIter = M == MODE_POLAR || M == MODE_POLAR_FAST;
-    PolarIter<M == MODE_POLAR_FAST> pe;
+    DeLoop<M> pe;
     for (;;) {
         const bool need = !done && i == kNone;
         const unsigned need_mask = __ballot_sync(0xFFFFFFFFu, need);
@@ -142,8 +109,8 @@ __global__ void __launch_bounds__(128) k_trace_queue(ShapeDev s, CameraDev c, ui
         if (done || i == kNone) continue;
         float de;
         if (kIter) {
-            if (!pe.advance(s)) continue;
-            de = pe.value();
+            if (pe.step(s)) continue;
+            de = pe.value(s);
         } else {
             de = eval<M>(s, c.eye[0] + t * d[0], c.eye[1] + t * d[1], c.eye[2] + t * d[2]);
         }
@@ -169,12 +136,12 @@ __global__ void __launch_bounds__(128) k_trace_queue(ShapeDev s, CameraDev c, ui
 
 // Sum over hit pixels of g[i] * dt_i/dtheta; with cap > 0, pixels whose
 // |dt_i/dtheta_k| exceeds cap for some k are left out.
+template <bool LONG>
 __global__ void __launch_bounds__(128) k_trace_backward(ShapeDev s, CameraDev c, Dm3 dm,
                                                         const float* __restrict__ depth,
                                                         const float* __restrict__ g, float cap,
                                                         float* __restrict__ params) {
     extern __shared__ __align__(16) float4 adj_smem[];
-    const AdjTape tape = adj_tape(adj_smem, s.max_iters, ADJ_CK);
     const uint32_t n = c.width * c.height;
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -183,8 +150,11 @@ __global__ void __launch_bounds__(128) k_trace_backward(ShapeDev s, CameraDev c,
         float d[3];
         pixel_ray(c, i, d);
         float o[8];
-        polar_de_grad<ADJ_CK>(s, dm.m, c.eye[0] + t * d[0], c.eye[1] + t * d[1],
-                              c.eye[2] + t * d[2], tape, o);
+        const float x = c.eye[0] + t * d[0], y = c.eye[1] + t * d[1], z = c.eye[2] + t * d[2];
+        if constexpr (LONG)
+            polar_de_grad_long(s, dm.m, x, y, z, reinterpret_cast<float*>(adj_smem), o);
+        else
+            polar_de_grad<ADJ_CK>(s, dm.m, x, y, z, adj_tape(adj_smem, s.max_iters, ADJ_CK), o);
         const float dn = o[1] * d[0] + o[2] * d[1] + o[3] * d[2];
         if (!(fabsf(dn) > 1e-6f)) continue;  // grazing ray: no stable depth derivative
         float dt[4];
@@ -368,13 +338,17 @@ cg_status cg_trace_backward_capped(const cg_shape* shape, const cg_camera* camer
     cudaStream_t st = (cudaStream_t)stream;
     CG_CUDA(cudaMemsetAsync(grad_params, 0, 4 * sizeof(float), st));
     const uint64_t n = (uint64_t)c.width * c.height;
+    const bool lng = shape->max_iters <= ADJ_LONG_MAX;
+    const unsigned B = lng ? ADJ_LONG_BLOCK : ADJ_BLOCK;
+    const size_t smem = lng ? long_tape_bytes(shape->max_iters, B)
+                            : adj_tape_bytes(shape->max_iters, ADJ_CK, B);
+    auto kernel = lng ? k_trace_backward<true> : k_trace_backward<false>;
     unsigned G = 0;
-    size_t smem = 0;
-    CG_TRY(adj_launch_shape(k_trace_backward, shape->max_iters, ADJ_CK, n, &G, &smem));
-    const uint32_t nwarps = G * 4;
+    CG_TRY(adj_launch_shape(kernel, B, smem, n, &G));
+    const uint32_t nwarps = G * (B / 32);
     float* partial = nullptr;
     CG_TRY(acquire_partials((size_t)nwarps * 4, st, &partial));
-    k_trace_backward<<<G, 128, smem, st>>>(s, c, dm, depth, grad_depth, cap, partial);
+    kernel<<<G, B, smem, st>>>(s, c, dm, depth, grad_depth, cap, partial);
     cg_status rs = cuda_status(cudaGetLastError(), "k_trace_backward", __FILE__, __LINE__);
     if (rs == CG_OK) rs = launch_sum_partials4(partial, nwarps, grad_params, st);
     const cg_status rr = release_partials(partial, st);
