@@ -23,7 +23,7 @@ template <int M>
 struct DeLoop {
     float px, py, pz;  // the point (polar forms: R^T p)
     float x, y, z, dr;
-    float r;           // |z|; MODE_P8: |z|^2
+    float r;           // |z|; MODE_P8: |z|^2; MODE_SPHERE: the distance
     uint32_t it;
     float limit;       // MODE_P8
     bool inside;       // MODE_P8
@@ -40,8 +40,16 @@ struct DeLoop {
         it = 0;
         if (M == MODE_P8) limit = p8_limit(s.p8_m2_max, py, pz);
     }
+    // A loop whose point, iterate and count were set by hand.
+    __device__ __forceinline__ void resume(const ShapeDev& s) {
+        if (M == MODE_P8) limit = p8_limit(s.p8_m2_max, py, pz);
+    }
     // One step; false when the loop has ended (max_iters >= 1).
     __device__ __forceinline__ bool step(const ShapeDev& s) {
+        if (M == MODE_SPHERE) {
+            r = sphere_de(s, px, py, pz);
+            return false;
+        }
         const bool last = ++it >= s.max_iters;
         if (M == MODE_P8) return p8_step(limit, px, py, pz, last, x, y, z, dr, r, inside);
         if (M == MODE_INT) return int_step(s, px, py, pz, last, x, y, z, dr, r);
@@ -50,9 +58,10 @@ struct DeLoop {
         if (M == MODE_INT_POLY)
             return int_poly_step(s.power, (float)s.power, s.bailout, px, py, pz, x, y, z, dr, r) &&
                    !last;
-        return polar_step_fast(s.power_f, s.bailout, px, py, pz, x, y, z, dr, r) && !last;
+        return polar_step_fast(s, px, py, pz, x, y, z, dr, r) && !last;
     }
     __device__ __forceinline__ float value(const ShapeDev& s) const {
+        if (M == MODE_SPHERE) return r;
         if (M == MODE_P8)
             return p8_value(s.max_iters, s.bailout, limit, px, py, pz, r, dr, inside);
         if (M == MODE_INT || M == MODE_POLAR) return de_value(r, dr);
