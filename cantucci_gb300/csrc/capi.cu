@@ -179,6 +179,8 @@ struct cg_mesher {
     cudaStream_t copy_stream = nullptr;  // host-output copies overlapping placement
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     cudaEvent_t fork = nullptr, join = nullptr;  // quads on copy_stream beside placement
+    cudaStream_t timing_stream = nullptr;        // a captured graph's timing events
+    cudaEvent_t timing_fork = nullptr;
     char* work = nullptr;
     size_t work_bytes = 0;
     cg_vertex* dverts = nullptr;
@@ -260,18 +262,23 @@ cg_status enqueue_mesh(cg_mesher* m, const ShapeDev& s, const SpanSetup& su, con
     if (dp)
         CG_CUDA(cudaMemcpyAsync(dp, m->gparams_host, sizeof(MeshGraphParams),
                                 cudaMemcpyHostToDevice, st));
-    CG_CUDA(record_event(m->ev[0], st));
+    cudaStream_t ts = m->timing_stream;
+    CG_CUDA(record_event(m->ev[0], st, ts, m->timing_fork));
     CG_CUDA(cudaMemsetAsync(w.sgn, 0, (size_t)d.n * d.n * d.W * sizeof(uint32_t), st));
     CG_TRY(launch_de_grid(s, make_grid(su, d.res), w.dists, m->numerics, st, w.sgn, d.W,
                           dp ? &dp->g : nullptr));
-    CG_CUDA(record_event(m->ev[1], st));
-    const SideStream side = {m->copy_stream, m->fork, m->join};
+    CG_CUDA(record_event(m->ev[1], st, ts, m->timing_fork));
+    const SideStream side = {m->copy_stream, m->fork, m->join, ts, m->timing_fork};
     PlaceOptions opt = place_options(m);
     opt.pp_dev = dp ? &dp->pp : nullptr;
     CG_TRY(launch_mesh_from_dists(s, su, d, w, dverts, vcap, didx, icap, st, m->ev[2],
                                   /*signs_ready=*/true, opt, &side));
-    CG_CUDA(record_event(m->ev[3], st));
+    CG_CUDA(record_event(m->ev[3], st, ts, m->timing_fork));
     CG_CUDA(cudaMemcpyAsync(m->hcnt, w.counters, sizeof(MeshCounters), cudaMemcpyDeviceToHost, st));
+    if (dp) {  // being captured: the timing events' stream joins the graph again
+        CG_CUDA(cudaEventRecord(m->timing_fork, ts));
+        CG_CUDA(cudaStreamWaitEvent(st, m->timing_fork, 0));
+    }
     return CG_OK;
 }
 
@@ -526,6 +533,12 @@ cg_status cg_mesher_create(int device, cg_mesher** out) {
     for (auto& e : m->ev) cudaEventCreate(&e);
     cudaEventCreateWithFlags(&m->fork, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&m->join, cudaEventDisableTiming);
+    cudaEventCreateWithFlags(&m->timing_fork, cudaEventDisableTiming);
+    if ((st = cuda_status(cudaStreamCreateWithFlags(&m->timing_stream, cudaStreamNonBlocking),
+                          "cudaStreamCreate", __FILE__, __LINE__)) != CG_OK) {
+        cg_mesher_destroy(m);
+        return st;
+    }
     int prio_lo = 0, prio_hi = 0;
     if (cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi) != cudaSuccess) prio_hi = prio_lo = 0;
     if ((st = cuda_status(cudaStreamCreateWithPriority(&m->copy_stream, cudaStreamNonBlocking,
@@ -560,6 +573,8 @@ void cg_mesher_destroy(cg_mesher* m) {
         if (e) cudaEventDestroy(e);
     if (m->fork) cudaEventDestroy(m->fork);
     if (m->join) cudaEventDestroy(m->join);
+    if (m->timing_fork) cudaEventDestroy(m->timing_fork);
+    if (m->timing_stream) cudaStreamDestroy(m->timing_stream);
     if (m->copy_stream) cudaStreamDestroy(m->copy_stream);
     if (m->stream) cudaStreamDestroy(m->stream);
     delete m;

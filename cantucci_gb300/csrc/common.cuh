@@ -81,12 +81,22 @@ __device__ __forceinline__ T* checked_at(T* p, uint64_t i, uint64_t n, unsigned 
 int sm_count();
 
 // A timing event: while `st` is being captured into a graph, recorded as an
-// event node of the graph (so it times the replay), else recorded now.
-inline cudaError_t record_event(cudaEvent_t ev, cudaStream_t st) {
+// event node of the graph (so it times the replay), else recorded now.  With
+// `side` the node goes to that stream, after what `st` holds so far (by way
+// of the event `fork`): an event node in the chain itself holds up the next
+// kernel by about 2 us.  The capture then has to join `side` again.
+inline cudaError_t record_event(cudaEvent_t ev, cudaStream_t st, cudaStream_t side = nullptr,
+                                cudaEvent_t fork = nullptr) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusActive)
-        return cudaEventRecordWithFlags(ev, st, cudaEventRecordExternal);
-    return cudaEventRecord(ev, st);
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusActive)
+        return cudaEventRecord(ev, st);
+    if (side) {
+        cudaError_t e = cudaEventRecord(fork, st);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(side, fork, 0);
+        if (e != cudaSuccess) return e;
+        st = side;
+    }
+    return cudaEventRecordWithFlags(ev, st, cudaEventRecordExternal);
 }
 
 // Grid size for a grid-stride kernel: enough blocks to fill every SM

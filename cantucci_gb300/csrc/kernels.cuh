@@ -96,8 +96,11 @@ struct MeshWork {
     MeshCounters* counters;
 };
 
+// res is a power of two (check_span_res), so rows and words split by shifts:
+// an integer division by a run-time value is some 20 instructions.
 struct MeshDims {
     uint32_t res, n, W, Wc;
+    uint32_t shift, wshift;  // log2 of res and of Wc
 };
 MeshDims mesh_dims(uint32_t res);
 // Byte size of a workspace for `res`; fills `w` with offsets from `base`.
@@ -136,9 +139,13 @@ struct PlaceOptions {
 // their capacity; counts land in w.counters.
 // A second stream and a fork / join event pair: with it the quad indices
 // are built concurrently with the vertex placement.
+// `timing` / `timing_fork`: where a captured graph records its timing events
+// (record_event).
 struct SideStream {
     cudaStream_t stream;
     cudaEvent_t fork, join;
+    cudaStream_t timing;
+    cudaEvent_t timing_fork;
 };
 cg_status launch_mesh_from_dists(const ShapeDev& s, const SpanSetup& su, const MeshDims& d,
                                  const MeshWork& w, cg_vertex* verts, uint64_t vcap,

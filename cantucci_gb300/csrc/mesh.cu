@@ -5,6 +5,8 @@
 #include <atomic>
 #include <cstring>
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "kernels.cuh"
 #include "mesh_rows.cuh"
@@ -19,6 +21,9 @@ MeshDims mesh_dims(uint32_t res) {
     d.n = res + 1;
     d.W = (d.n + 31) / 32;
     d.Wc = (res + 31) / 32;
+    for (d.shift = 0; (2u << d.shift) <= res; ++d.shift) {
+    }
+    d.wshift = d.shift > 5 ? d.shift - 5 : 0;
     return d;
 }
 
@@ -78,9 +83,9 @@ struct RowLanes {
     __device__ RowLanes(const MeshDims& d) {
         const uint32_t lane = threadIdx.x & 31;
         L = d.Wc;
-        per_warp = 32 / L;
-        sub = lane % L;
-        lane_row = lane / L;
+        per_warp = 32u >> d.wshift;
+        sub = lane & (L - 1);
+        lane_row = lane >> d.wshift;
         warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
         nwarps = (gridDim.x * blockDim.x) >> 5;
     }
@@ -142,12 +147,82 @@ __global__ void __launch_bounds__(256) k_vertex_list(MeshDims d, const uint32_t*
     }
 }
 
+// Spans up to res 64: k_cells, k_vertex_list, k_quad_count and both scans in
+// one launch of one cluster, a cell word to a thread.  The words are in row
+// order, so one scan over them (in the CTA, then over the cluster's totals
+// through distributed shared memory) gives every word's first vertex id and,
+// beside it, every row's first quad.  Latency-bound either way; six launches
+// became one (a res-64 leaf's mesh 71 -> 62 us with the timing events off the
+// path).
+constexpr uint32_t kClusterRowsMaxRes = 64;
+constexpr unsigned kRowsCluster = 8;
+
+__global__ void __cluster_dims__(kRowsCluster, 1, 1) __launch_bounds__(1024)
+    k_rows_cluster(const uint32_t* __restrict__ sgn, MeshDims d, uint32_t* __restrict__ cellbits,
+                   uint32_t* __restrict__ wordoff, uint32_t* __restrict__ rowoff,
+                   uint32_t* __restrict__ quadoff, uint32_t* __restrict__ cellidx,
+                   MeshCounters* __restrict__ cnt) {
+    namespace cgr = cooperative_groups;
+    __shared__ uint32_t ws[33];
+    __shared__ uint2 totals[kRowsCluster];  // (vertices, quads) of every CTA
+    cgr::cluster_group cluster = cgr::this_cluster();
+    const uint32_t rank = cluster.block_rank();
+    const uint32_t rows = d.res * d.res, words = rows << d.wshift;
+    [[maybe_unused]] const uint64_t cap = (uint64_t)rows * d.res;
+    const uint32_t u = rank * blockDim.x + threadIdx.x;
+    const bool ok = u < words;
+    const uint32_t r = u >> d.wshift, w = u & (d.Wc - 1);
+    uint32_t surf = 0, quads = 0;
+    if (ok) {
+        surf = cells_word(sgn, d, r, w);
+        const EdgeWords e = edge_words(sgn, d, r >> d.shift, r & (d.res - 1), w);
+        quads = __popc(e.ex) + __popc(e.ey) + __popc(e.ez);
+    }
+    uint32_t vtot, qtot;
+    uint32_t v = block_exclusive_scan(__popc(surf), ws, vtot);
+    uint32_t q = block_exclusive_scan(quads, ws, qtot);
+    if (threadIdx.x < kRowsCluster)
+        *cluster.map_shared_rank(&totals[rank], threadIdx.x) = make_uint2(vtot, qtot);
+    cluster.sync();
+    uint2 all = make_uint2(0u, 0u);
+#pragma unroll
+    for (uint32_t k = 0; k < kRowsCluster; ++k) {
+        const uint2 t = totals[k];
+        v += k < rank ? t.x : 0u;
+        q += k < rank ? t.y : 0u;
+        all.x += t.x;
+        all.y += t.y;
+    }
+    // The row's first vertex is that of its word 0, in this warp (Wc <= 2).
+    const uint32_t row_v = __shfl_sync(0xFFFFFFFFu, v, (threadIdx.x & 31) & ~(d.Wc - 1));
+    if (ok) {
+        CG_AT(cellbits, u, words) = surf;
+        CG_AT(wordoff, u, words) = v - row_v;
+        if (w == 0) {
+            CG_AT(rowoff, r, rows) = v;
+            CG_AT(quadoff, r, rows) = q;
+        }
+        while (surf) {
+            const uint32_t b = __ffs(surf) - 1;
+            surf &= surf - 1;
+            CG_AT(cellidx, v, cap) = r * d.res + w * 32 + b;
+            ++v;
+        }
+    }
+    if (rank == 0 && threadIdx.x == 0) {
+        cnt->vertices = all.x;
+        cnt->quads = all.y;
+        cnt->status = 0;
+        cnt->edges = 0;
+    }
+}
+
 // One vertex per thread (buffer.rs:149-274).  A warp places 32 consecutive
 // vertices and stores them through shared memory as 16-byte chunks (32
 // vertices = 896 bytes = 56 float4), so the stores are coalesced whether
 // `verts` is device memory or pinned host memory written over the C2C link.
 template <int M, bool AN, bool ROOT, bool QEF>
-__global__ void __launch_bounds__(128) k_place(ShapeDev s, PlaceParams pp, MeshDims d,
+__global__ void __launch_bounds__(128, (AN || QEF) ? 5 : (ROOT ? 1 : 9)) k_place(ShapeDev s, PlaceParams pp, MeshDims d,
                                                const float* __restrict__ dists,
                                                const uint32_t* __restrict__ cellidx,
                                                MeshCounters* __restrict__ cnt,
@@ -198,11 +273,18 @@ __global__ void __launch_bounds__(128) k_place(ShapeDev s, PlaceParams pp, MeshD
     if (bad) atomicOr(&cnt->status, MESH_LERP_FAIL);
 }
 
-// Small spans: the seven samples of a vertex on seven lanes of a group of
-// eight (four vertices per warp), so a vertex waits for one estimator call
-// instead of seven in a row; lane 0 of the group forms the record.  The
-// same operations as k_place<M, false, false, false>, so the same bits.
-// The loop bound is warp-uniform, so every lane reaches the shuffles.
+// Small spans: a warp takes `per` vertices, forms their positions on `per`
+// lanes, and then evaluates their 7 per samples 32 at a time, so a vertex
+// waits for one estimate per round instead of seven in a row.  With few
+// vertices in the span a warp takes 4 (28 samples, one round: the shortest
+// chain); from kSpreadTwoRounds on it takes 9 (63 samples, two rounds), which
+// shares the twelve crossings of a cell's edges among more samples and leaves
+// one lane idle in 64 (a res-64 leaf of 30 K vertices: 23.5 -> 17 us against
+// eight lanes per vertex, each forming the position).  The same operations as
+// k_place<M, false, false, false>, so the same bits.  The loop bound is
+// warp-uniform.
+constexpr uint32_t kSpreadTwoRounds = 8192;
+
 template <int M>
 __global__ void __launch_bounds__(128) k_place_spread(ShapeDev s, PlaceParams pp, MeshDims d,
                                                       const float* __restrict__ dists,
@@ -212,39 +294,54 @@ __global__ void __launch_bounds__(128) k_place_spread(ShapeDev s, PlaceParams pp
                                                       uint64_t vcap,
                                                       const PlaceParams* __restrict__ ppp) {
     if (ppp) pp = *ppp;
+    __shared__ float stage[4][64];  // per warp: sample distances, then records
     const uint32_t V = cnt->vertices;
-    const uint32_t lane = threadIdx.x & 31, k = lane & 7, g0 = lane & ~7u;
+    const uint32_t per = V < kSpreadTwoRounds ? 4u : 9u;
+    const uint32_t lane = threadIdx.x & 31;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    float* st = stage[threadIdx.x >> 5];
     float* vf = reinterpret_cast<float*>(verts);
     bool bad = false;
-    for (uint32_t base = warp * 4; base < V; base += nwarps * 4) {
-        const uint32_t v = base + (lane >> 3);
-        const bool live = v < V;
-        float vx = 0.0f, vy = 0.0f, vz = 0.0f, val = 0.0f;
-        if (live) {
+    for (uint32_t base = warp * per; base < V; base += nwarps * per) {
+        const uint32_t left = V - base < per ? V - base : per;
+        float vx = 0.0f, vy = 0.0f, vz = 0.0f;
+        if (lane < left) {
             CellCrossings cc;
-            cell_crossings(pp, d, dists, CG_AT(cellidx, v, (uint64_t)d.res * d.res * d.res), cc);
+            cell_crossings(pp, d, dists,
+                           CG_AT(cellidx, base + lane, (uint64_t)d.res * d.res * d.res), cc);
             const float cf = (float)cc.count;
             vx = __fadd_rn(0.0f, __fdiv_rn(cc.sx, cf));
             vy = __fadd_rn(0.0f, __fdiv_rn(cc.sy, cf));
             vz = __fadd_rn(0.0f, __fdiv_rn(cc.sz, cf));
-            if (k == 0) bad |= cc.bad;
-            if (k < 7) {
+            bad |= cc.bad;
+        }
+        for (uint32_t i0 = 0; i0 < 7 * left; i0 += 32) {
+            const uint32_t i = i0 + lane, j = i / 7, k = i - 7 * j;  // sample k of vertex j
+            const float ax = __shfl_sync(0xFFFFFFFFu, vx, j & 31);
+            const float ay = __shfl_sync(0xFFFFFFFFu, vy, j & 31);
+            const float az = __shfl_sync(0xFFFFFFFFu, vz, j & 31);
+            if (i < 7 * left) {
                 float qx, qy, qz;
-                sample_point(pp, (int)k, vx, vy, vz, qx, qy, qz);
-                val = eval<M>(s, qx, qy, qz);
+                sample_point(pp, (int)k, ax, ay, az, qx, qy, qz);
+                st[i] = eval<M>(s, qx, qy, qz);
             }
         }
-        float de[7];
+        __syncwarp();
+        if (lane < left) {
+            float de[7], o[7];
 #pragma unroll
-        for (int j = 0; j < 7; ++j) de[j] = __shfl_sync(0xFFFFFFFFu, val, g0 + j);
-        if (live && k == 0 && v < vcap) {
-            float o[7];
+            for (int k = 0; k < 7; ++k) de[k] = st[7 * lane + k];
             vertex_record(de, vx, vy, vz, o);
 #pragma unroll
-            for (int j = 0; j < 7; ++j) CG_AT(vf, (uint64_t)v * 7 + j, vcap * 7) = o[j];
+            for (int k = 0; k < 7; ++k) st[7 * lane + k] = o[k];
         }
+        __syncwarp();
+        const uint64_t room = base < vcap ? vcap - base : 0;
+        const uint32_t words = 7 * (left < room ? left : (uint32_t)room);
+        for (uint32_t i = lane; i < words; i += 32)
+            CG_AT(vf, (uint64_t)base * 7 + i, vcap * 7) = st[i];
+        __syncwarp();
     }
     if (bad) atomicOr(&cnt->status, MESH_LERP_FAIL);
 }
@@ -324,7 +421,7 @@ __global__ void __launch_bounds__(256) k_edge_list(const uint32_t* __restrict__ 
 // zero of the linear interpolant of its corner distances) and the DE's
 // gradient there.
 template <int M, bool ROOT>
-__global__ void __launch_bounds__(128) k_edge_data(ShapeDev s, PlaceParams pp, MeshDims d,
+__global__ void __launch_bounds__(128, 5) k_edge_data(ShapeDev s, PlaceParams pp, MeshDims d,
                                                    const float* __restrict__ dists,
                                                    const uint32_t* __restrict__ list,
                                                    const MeshCounters* __restrict__ cnt,
@@ -396,7 +493,8 @@ __global__ void __launch_bounds__(256) k_quad_emit_fine(const uint32_t* __restri
     const uint32_t lane = threadIdx.x & 31, bit = 1u << lane;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < units; u += nwarps) {
-        const uint32_t r = u / d.Wc, w = u % d.Wc, x = r / d.res, y = r % d.res;
+        const uint32_t r = u >> d.wshift, w = u & (d.Wc - 1);
+        const uint32_t x = r >> d.shift, y = r & (d.res - 1);
         uint64_t q = CG_AT(quadoff, r, rows);
         for (uint32_t w2 = 0; w2 < w; ++w2) {
             const EdgeWords e2 = edge_words(sgn, d, x, y, w2);
@@ -444,10 +542,10 @@ __global__ void __launch_bounds__(256) k_points_table(MeshDims d,
     const uint32_t total = d.res * d.res * d.res;
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < total;
          c += gridDim.x * blockDim.x) {
-        const uint32_t z = c % d.res, r = c / d.res;
+        const uint32_t z = c & (d.res - 1), r = c >> d.shift;
         const uint32_t word = CG_AT(cellbits, r * d.Wc + (z >> 5), (uint64_t)d.res * d.res * d.Wc);
         CG_AT(points, c, total) = ((word >> (z & 31)) & 1u)
-                        ? vertex_id(d, cellbits, wordoff, rowoff, r / d.res, r % d.res, z)
+                        ? vertex_id(d, cellbits, wordoff, rowoff, r >> d.shift, r & (d.res - 1), z)
                         : 0xFFFFFFFFu;
     }
 }
@@ -658,7 +756,8 @@ static cg_status launch_place(const ShapeDev& s, const SpanSetup& su, const Mesh
     return CG_OK;
 }
 
-// Surface cells, their scan and the vertex list (step 2 up to placement).
+// Surface cells, their scan and the vertex list (step 2 up to placement); for
+// spans up to res 64 the quad counts and their scan too.
 static cg_status launch_cells(const MeshDims& d, const MeshWork& w, cudaStream_t st,
                               bool signs_ready) {
     const uint32_t rows = d.res * d.res;
@@ -667,6 +766,14 @@ static cg_status launch_cells(const MeshDims& d, const MeshWork& w, cudaStream_t
         const unsigned B = 256, G = grid_for(warps * 32, B, 8);
         k_sign_words<<<G, B, 0, st>>>(w.dists, d.n, d.W, w.sgn);
         CG_CHECK_LAUNCH("k_sign_words");
+    }
+    if (d.res <= kClusterRowsMaxRes) {
+        const uint32_t words = rows << d.wshift;
+        unsigned B = ((words + kRowsCluster - 1) / kRowsCluster + 31) & ~31u;
+        k_rows_cluster<<<kRowsCluster, B, 0, st>>>(w.sgn, d, w.cellbits, w.wordoff, w.rowoff,
+                                                   w.quadoff, w.cellidx, w.counters);
+        CG_CHECK_LAUNCH("k_rows_cluster");
+        return CG_OK;
     }
     {
         const unsigned B = 256, G = grid_for(row_lanes(d), B, 8);
@@ -683,6 +790,7 @@ static cg_status launch_cells(const MeshDims& d, const MeshWork& w, cudaStream_t
 }
 
 static cg_status launch_quad_count(const MeshDims& d, const MeshWork& w, cudaStream_t st) {
+    if (d.res <= kClusterRowsMaxRes) return CG_OK;  // counted with the cells
     const uint32_t rows = d.res * d.res;
     const unsigned B = 256, G = grid_for(rows, B, 8);
     k_quad_count<<<G, B, 0, st>>>(w.sgn, d, w.quadcnt);
@@ -734,7 +842,8 @@ cg_status launch_mesh_from_dists(const ShapeDev& s, const SpanSetup& su, const M
         CG_CUDA(cudaEventRecord(side->join, side->stream));
         if (opt.qef) CG_TRY(edge_table(&et));
         CG_TRY(launch_place(s, su, d, w, verts, vcap, st, opt, et));
-        if (ev_after_vertices) CG_CUDA(record_event(ev_after_vertices, st));
+        if (ev_after_vertices)
+            CG_CUDA(record_event(ev_after_vertices, st, side->timing, side->timing_fork));
         CG_CUDA(cudaStreamWaitEvent(st, side->join, 0));
         return CG_OK;
     }

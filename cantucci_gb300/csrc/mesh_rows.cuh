@@ -40,7 +40,7 @@ __device__ __forceinline__ uint32_t sign_hi(const uint32_t* __restrict__ sgn, co
 // cell crosses iff the sign bits of its 8 corners are not all equal.
 __device__ __forceinline__ uint32_t cells_word(const uint32_t* __restrict__ sgn, const MeshDims& d,
                                                uint32_t r, uint32_t w) {
-    const uint32_t x = r / d.res, y = r % d.res;
+    const uint32_t x = r >> d.shift, y = r & (d.res - 1);
     const uint32_t r00 = x * d.n + y, r01 = r00 + 1, r10 = r00 + d.n, r11 = r10 + 1;
     [[maybe_unused]] const uint64_t ns = (uint64_t)d.n * d.n * d.W;
     const uint32_t a0 = CG_AT(sgn, r00 * d.W + w, ns), a1 = CG_AT(sgn, r01 * d.W + w, ns);
@@ -254,10 +254,9 @@ struct CellCrossings {
 __device__ __forceinline__ void cell_crossings(const PlaceParams& pp, const MeshDims& d,
                                                const float* __restrict__ dists, uint32_t c,
                                                CellCrossings& q) {
-    q.z = c % d.res;
-    const uint32_t xy = c / d.res;
-    q.y = xy % d.res;
-    q.x = xy / d.res;
+    q.z = c & (d.res - 1);
+    q.y = (c >> d.shift) & (d.res - 1);
+    q.x = c >> (2 * d.shift);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
         const uint32_t cx = q.x + ((k >> 2) & 1), cy = q.y + ((k >> 1) & 1), cz = q.z + (k & 1);
@@ -453,7 +452,7 @@ __device__ __forceinline__ EdgeWords edge_words(const uint32_t* __restrict__ sgn
 
 __device__ __forceinline__ uint32_t quad_count_row(const uint32_t* __restrict__ sgn,
                                                    const MeshDims& d, uint32_t r) {
-    const uint32_t x = r / d.res, y = r % d.res;
+    const uint32_t x = r >> d.shift, y = r & (d.res - 1);
     uint32_t c = 0;
     for (uint32_t w = 0; w < d.Wc; ++w) {
         const EdgeWords e = edge_words(sgn, d, x, y, w);
@@ -537,7 +536,7 @@ __device__ __forceinline__ void quad_emit_row(const uint32_t* __restrict__ sgn, 
                                               const uint32_t* __restrict__ rowoff, uint32_t vbase,
                                               uint64_t q, uint32_t* __restrict__ idx, uint64_t icap,
                                               uint32_t r) {
-    const uint32_t x = r / d.res, y = r % d.res;
+    const uint32_t x = r >> d.shift, y = r & (d.res - 1);
     for (uint32_t w = 0; w < d.Wc; ++w)
         q = quad_emit_word(edge_words(sgn, d, x, y, w), d, dists, cellbits, wordoff, rowoff, vbase,
                            q, idx, icap, x, y, w);

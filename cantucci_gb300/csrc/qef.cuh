@@ -41,12 +41,18 @@ __device__ __forceinline__ D3 d3mul(const D3& a, const D3& b) {
 __device__ __forceinline__ D3 d3scale(float c, const D3& a) {
     return {__fmul_rn(c, a.v), c * a.d0, c * a.d1, c * a.d2};
 }
+// NORMAL: operands in the range of the shortened operations (p8_step's test);
+// the same bits.
+template <bool NORMAL>
 __device__ __forceinline__ D3 d3div(const D3& a, const D3& b) {
-    const float q = __fdiv_rn(a.v, b.v), inv = 1.0f / b.v;
+    const float q = NORMAL ? div_rn_normal(a.v, b.v) : __fdiv_rn(a.v, b.v);
+    const float inv = NORMAL ? rcp_rn_normal(b.v) : 1.0f / b.v;
     return {q, (a.d0 - q * b.d0) * inv, (a.d1 - q * b.d1) * inv, (a.d2 - q * b.d2) * inv};
 }
+template <bool NORMAL>
 __device__ __forceinline__ D3 d3sqrt(const D3& a) {
-    const float s = __fsqrt_rn(a.v), h = 0.5f / s;
+    const float s = NORMAL ? sqrt_rn_normal(a.v) : __fsqrt_rn(a.v);
+    const float h = NORMAL ? 0.5f * rcp_rn_normal(s) : 0.5f / s;
     return {s, a.d0 * h, a.d1 * h, a.d2 * h};
 }
 
@@ -59,34 +65,44 @@ __device__ __forceinline__ D3 d3sqrt(const D3& a) {
 // whose derivative is 8 r^7 r'.  g[0] = DE (the estimator's bits), g[1..3] =
 // dDE/dp; DE' = 0.5 (ln r + 1) r' / dr - DE dr' / dr at the returned (stale
 // or escaping) r.
-static __device__ __noinline__ void p8_de_gradient(uint32_t max_iters, float bailout, float px,
-                                                   float py, float pz, float* g) {
+// NORMAL: with the range tests of p8_step, false for a point that they do not
+// cover (g is then not written); else with the IEEE operations throughout.
+template <bool NORMAL>
+__device__ __forceinline__ bool p8_gradient_loop(uint32_t max_iters, float bailout, float m2_max,
+                                                 float px, float py, float pz, float* g) {
     const D3 qx = {px, 1.0f, 0.0f, 0.0f}, qy = {py, 0.0f, 1.0f, 0.0f}, qz = {pz, 0.0f, 0.0f, 1.0f};
     D3 x = qx, y = qy, z = qz, dr = d3c(1.0f), r = d3c(0.0f);
-    for (uint32_t i = 0; i < max_iters; ++i) {
-        r = d3sqrt(d3add(d3add(d3mul(x, x), d3mul(y, y)), d3mul(z, z)));
-        if (r.v > bailout) break;
+    for (uint32_t i = 0; i < max_iters;) {
+        const D3 x2 = d3mul(x, x), y2 = d3mul(y, y), z2 = d3mul(z, z);
+        const D3 rxy2 = d3add(x2, y2), m2 = d3add(rxy2, z2);
+        bool out = false;
+        if (NORMAL) {
+            out = m2.v > m2_max;
+            if (!out && !(m2.v <= m2_max && rxy2.v >= kP8MinRxy2)) return false;
+        }
+        r = NORMAL && !out ? d3sqrt<true>(m2) : d3sqrt<false>(m2);
+        if (NORMAL ? out : r.v > bailout) break;
         // f32::powi(r, 7) = (r * r^2) * r^4, times P, times dr, plus 1
         const D3 r2 = d3mul(r, r), r4 = d3mul(r2, r2), r7 = d3mul(d3mul(r, r2), r4);
         dr = d3add(d3mul(d3scale(8.0f, r7), dr), d3c(1.0f));
+        if (++i == max_iters) break;  // nobody reads the last z
         D3 nx, ny, nz;
-        if (on_z_axis(x.v, y.v)) {
+        if (!NORMAL && on_z_axis(x.v, y.v)) {
             nx = d3c(0.0f);
             ny = d3c(0.0f);
             const float k = 8.0f * r7.v;
             nz = {rotate_axis_z<Exact>(8, x.v, y.v, z.v), k * r.d0, k * r.d1, k * r.d2};
         } else {
-            const D3 x2 = d3mul(x, x), x4 = d3mul(x2, x2), x6 = d3mul(x4, x2), x8 = d3mul(x4, x4);
-            const D3 y2 = d3mul(y, y), y4 = d3mul(y2, y2), y6 = d3mul(y4, y2), y8 = d3mul(y4, y4);
-            const D3 z2 = d3mul(z, z), z4 = d3mul(z2, z2), z6 = d3mul(z4, z2), z8 = d3mul(z4, z4);
-            const D3 rxy2 = d3add(x2, y2);
+            const D3 x4 = d3mul(x2, x2), x6 = d3mul(x4, x2), x8 = d3mul(x4, x4);
+            const D3 y4 = d3mul(y2, y2), y6 = d3mul(y4, y2), y8 = d3mul(y4, y4);
+            const D3 z4 = d3mul(z2, z2), z6 = d3mul(z4, z2), z8 = d3mul(z4, z4);
             const D3 rxy4 = d3mul(rxy2, rxy2);
             const D3 rxy6 = d3mul(rxy2, rxy4);
             const D3 rxy8 = d3mul(rxy4, rxy4);
             const D3 num = d3sub(d3add(d3sub(z8, d3mul(d3scale(28.0f, z6), rxy2)),
                                        d3mul(d3scale(70.0f, z4), rxy4)),
                                  d3mul(d3scale(28.0f, z2), rxy6));
-            const D3 a = d3add(d3c(1.0f), d3div(num, rxy8));
+            const D3 a = d3add(d3c(1.0f), d3div<NORMAL>(num, rxy8));
             const D3 X = d3sub(d3sub(d3add(d3sub(x8, d3mul(d3scale(28.0f, x6), y2)),
                                            d3mul(d3scale(70.0f, x4), y4)),
                                      d3mul(d3scale(28.0f, x2), y6)),
@@ -97,7 +113,7 @@ static __device__ __noinline__ void p8_de_gradient(uint32_t max_iters, float bai
                                y6);
             ny = d3mul(d3mul(d3mul(d3scale(8.0f, a), x), y), Y);
             const D3 Z = d3add(d3sub(z4, d3mul(d3scale(6.0f, z2), rxy2)), rxy4);
-            nz = d3mul(d3mul(d3mul(d3scale(8.0f, z), d3sqrt(rxy2)), d3sub(z2, rxy2)), Z);
+            nz = d3mul(d3mul(d3mul(d3scale(8.0f, z), d3sqrt<NORMAL>(rxy2)), d3sub(z2, rxy2)), Z);
         }
         x = d3add(nx, qx);
         y = d3add(ny, qy);
@@ -110,6 +126,18 @@ static __device__ __noinline__ void p8_de_gradient(uint32_t max_iters, float bai
     g[1] = c_r * r.d0 + c_dr * dr.d0;
     g[2] = c_r * r.d1 + c_dr * dr.d1;
     g[3] = c_r * r.d2 + c_dr * dr.d2;
+    return true;
+}
+
+static __device__ __noinline__ void p8_gradient_special(uint32_t max_iters, float bailout, float px,
+                                                        float py, float pz, float* g) {
+    p8_gradient_loop<false>(max_iters, bailout, 0.0f, px, py, pz, g);
+}
+
+static __device__ __noinline__ void p8_de_gradient(uint32_t max_iters, float bailout, float m2_max,
+                                                   float px, float py, float pz, float* g) {
+    if (!p8_gradient_loop<true>(max_iters, bailout, m2_max, px, py, pz, g))
+        p8_gradient_special(max_iters, bailout, px, py, pz, g);
 }
 
 // DE and dDE/dp of the shape in g[0..3], one forward-mode pass:
@@ -132,7 +160,7 @@ __device__ __forceinline__ void shape_gradient(const ShapeDev& s, float x, float
         g[2] = dy * inv;
         g[3] = dz * inv;
     } else if constexpr (M == MODE_P8 || M == MODE_P8_IT15 || M == MODE_P8_FAST) {
-        p8_de_gradient(s.max_iters, s.bailout, x, y, z, g);
+        p8_de_gradient(s.max_iters, s.bailout, s.p8_m2_max, x, y, z, g);
     } else {
         float o[5];
         if constexpr (M == MODE_INT || M == MODE_INT_POLY) {
