@@ -97,6 +97,36 @@ __global__ void __launch_bounds__(256) k_de_grid(ShapeDev s, GridDev g, float* _
     }
 }
 
+// Small grids, one 2x4x4 brick of corners per warp and one warp's work per
+// warp: k_de_grid_brick's lanes without its walk, in fewer registers.
+template <int M>
+__global__ void __launch_bounds__(128, 10) k_de_grid_small(ShapeDev s, GridDev g,
+                                                           float* __restrict__ out,
+                                                           uint32_t* __restrict__ sgn, uint32_t W,
+                                                           const GridDev* __restrict__ gp) {
+    if (gp) g = *gp;
+    const uint32_t n = g.n, lane = threadIdx.x & 31;
+    const uint32_t BX = (n + 1) >> 1, B4 = (n + 3) >> 2;
+    const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t t = b / B4, bx = t / B4;
+    if (bx >= BX) return;
+    const uint32_t x = 2 * bx + (lane >> 4), y = 4 * (t - bx * B4) + ((lane >> 2) & 3),
+                   z = 4 * (b - t * B4) + (lane & 3);
+    bool pos = false;
+    const bool in = x < n && y < n && z < n;
+    if (in) {
+        const float d = eval<M>(s, grid_coord(g, 0, x), grid_coord(g, 1, y), grid_coord(g, 2, z));
+        CG_AT(out, ((size_t)x * n + y) * n + z, (uint64_t)n * n * n) = d;
+        pos = (__float_as_uint(d) >> 31) == 0u;
+    }
+    if (sgn) {
+        const uint32_t bits = __ballot_sync(0xFFFFFFFFu, pos) >> (lane & ~3u) & 0xFu;
+        if ((lane & 3) == 0 && bits)
+            atomicOr(&CG_AT(sgn, (x * n + y) * W + (z >> 5), (uint64_t)n * n * W),
+                     bits << (z & 31));
+    }
+}
+
 // Large grids: each warp evaluates 2x4x4 bricks of corners (x, y, z), which
 // keeps the escape counts of a warp's lanes close (89% lane efficiency on the
 // 513^3 span vs 75% for 32 corners along z).  A work unit is a run of
@@ -390,13 +420,15 @@ static void launch_grid_mode(const ShapeDev& s, const GridDev& g, float* out, ui
                              uint32_t W, cudaStream_t st, const GridDev* gp) {
     const unsigned B = 256;
     int k = g_de_grid_kernel;
-    // Up to 65^3 corners (res 64, cantucci's leaves) one corner per thread:
-    // a warp's DE chain is then the whole time (about 12 us for one
-    // 15-iteration evaluation at low occupancy), and the linear kernel's 45
-    // registers (5 resident blocks per SM) fit the grid in fewer waves than
-    // the bricks' 72 (3 blocks): 19.6 against 23.5 us for the res-64 grid.
+    // Up to 65^3 corners (res 64, cantucci's leaves) one brick to a warp: the
+    // brick walk's 63 registers (4 blocks of 256 threads per SM) would fit the
+    // grid in more waves than k_de_grid_small's 44, and one corner per thread
+    // in row order keeps 24 lanes busy against 27 (15.8 against 14.7 us).
     if (k == DE_GRID_AUTO) k = g.n > 65 ? DE_GRID_BRICK : DE_GRID_LINEAR;
-    if (k == DE_GRID_PACKED && (M == MODE_P8 || M == MODE_P8_IT15)) {
+    if (g_de_grid_kernel == DE_GRID_AUTO && k == DE_GRID_LINEAR) {
+        const uint64_t b4 = (g.n + 3) >> 2, bricks = ((g.n + 1) >> 1) * b4 * b4;
+        k_de_grid_small<M><<<(unsigned)((bricks + 3) / 4), 128, 0, st>>>(s, g, out, sgn, W, gp);
+    } else if (k == DE_GRID_PACKED && (M == MODE_P8 || M == MODE_P8_IT15)) {
         const uint64_t b4 = (g.n + 3) >> 2;
         k_de_grid_p8x2<<<grid_for(b4 * b4 * b4 * 32, B, 8), B, 0, st>>>(s, g, out, sgn, W, gp);
     } else if (k != DE_GRID_LINEAR) {

@@ -155,9 +155,10 @@ __global__ void __launch_bounds__(256) k_vertex_list(MeshDims d, const uint32_t*
 // became one (a res-64 leaf's mesh 71 -> 62 us with the timing events off the
 // path).
 constexpr uint32_t kClusterRowsMaxRes = 64;
-constexpr unsigned kRowsCluster = 8;
+// (16 CTAs: a cluster of 8 with 1024 threads each took 9.5 us, this 7.)
+constexpr unsigned kRowsCluster = 16;
 
-__global__ void __cluster_dims__(kRowsCluster, 1, 1) __launch_bounds__(1024)
+__global__ void __cluster_dims__(kRowsCluster, 1, 1) __launch_bounds__(512)
     k_rows_cluster(const uint32_t* __restrict__ sgn, MeshDims d, uint32_t* __restrict__ cellbits,
                    uint32_t* __restrict__ wordoff, uint32_t* __restrict__ rowoff,
                    uint32_t* __restrict__ quadoff, uint32_t* __restrict__ cellidx,
@@ -178,11 +179,14 @@ __global__ void __cluster_dims__(kRowsCluster, 1, 1) __launch_bounds__(1024)
         const EdgeWords e = edge_words(sgn, d, r >> d.shift, r & (d.res - 1), w);
         quads = __popc(e.ex) + __popc(e.ey) + __popc(e.ez);
     }
-    uint32_t vtot, qtot;
-    uint32_t v = block_exclusive_scan(__popc(surf), ws, vtot);
-    uint32_t q = block_exclusive_scan(quads, ws, qtot);
+    // At most 32 vertices and 96 quads a word: the sums over a CTA's 512 words
+    // take 16 bits each, one scan does both.
+    uint32_t both;
+    const uint32_t vq = block_exclusive_scan(__popc(surf) | quads << 16, ws, both);
+    uint32_t v = vq & 0xFFFFu, q = vq >> 16;
     if (threadIdx.x < kRowsCluster)
-        *cluster.map_shared_rank(&totals[rank], threadIdx.x) = make_uint2(vtot, qtot);
+        *cluster.map_shared_rank(&totals[rank], threadIdx.x) =
+            make_uint2(both & 0xFFFFu, both >> 16);
     cluster.sync();
     uint2 all = make_uint2(0u, 0u);
 #pragma unroll
@@ -769,7 +773,10 @@ static cg_status launch_cells(const MeshDims& d, const MeshWork& w, cudaStream_t
     }
     if (d.res <= kClusterRowsMaxRes) {
         const uint32_t words = rows << d.wshift;
-        unsigned B = ((words + kRowsCluster - 1) / kRowsCluster + 31) & ~31u;
+        static const cudaError_t cluster16 = cudaFuncSetAttribute(
+            k_rows_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        CG_CUDA(cluster16);
+        const unsigned B = ((words + kRowsCluster - 1) / kRowsCluster + 31) & ~31u;
         k_rows_cluster<<<kRowsCluster, B, 0, st>>>(w.sgn, d, w.cellbits, w.wordoff, w.rowoff,
                                                    w.quadoff, w.cellidx, w.counters);
         CG_CHECK_LAUNCH("k_rows_cluster");
