@@ -4,6 +4,7 @@
 
 #include "common.cuh"
 #include "de.cuh"
+#include "grid_units.cuh"
 #include "kernels.cuh"
 #include "lane_pool.cuh"
 #include "point_io.cuh"
@@ -97,98 +98,128 @@ __global__ void __launch_bounds__(256) k_de_grid(ShapeDev s, GridDev g, float* _
     }
 }
 
-// Small grids, one 2x4x4 brick of corners per warp and one warp's work per
-// warp: k_de_grid_brick's lanes without its walk, in fewer registers.
+struct GridCoord {
+    const GridDev& g;
+    __device__ __forceinline__ float operator()(int k, uint32_t v) const {
+        return grid_coord(g, k, v);
+    }
+};
+
+// Grids of res 32 and 64, one brick or face item to a warp: the lanes of
+// k_de_grid_units without its walk, in fewer registers.
 template <int M>
 __global__ void __launch_bounds__(128, 10) k_de_grid_small(ShapeDev s, GridDev g,
                                                            float* __restrict__ out,
                                                            uint32_t* __restrict__ sgn, uint32_t W,
+                                                           uint32_t shift,
                                                            const GridDev* __restrict__ gp) {
     if (gp) g = *gp;
+    const GridCoord coord{g};
     const uint32_t n = g.n, lane = threadIdx.x & 31;
-    const uint32_t BX = (n + 1) >> 1, B4 = (n + 3) >> 2;
-    const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t t = b / B4, bx = t / B4;
-    if (bx >= BX) return;
-    const uint32_t x = 2 * bx + (lane >> 4), y = 4 * (t - bx * B4) + ((lane >> 2) & 3),
-                   z = 4 * (b - t * B4) + (lane & 3);
-    bool pos = false;
-    const bool in = x < n && y < n && z < n;
-    if (in) {
-        const float d = eval<M>(s, grid_coord(g, 0, x), grid_coord(g, 1, y), grid_coord(g, 2, z));
-        CG_AT(out, ((size_t)x * n + y) * n + z, (uint64_t)n * n * n) = d;
-        pos = (__float_as_uint(d) >> 31) == 0u;
+    const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, bricks = core_bricks(shift);
+    if (c >= bricks) {
+        if (c - bricks < face_items(shift)) face_item<M>(s, coord, shift, W, c - bricks, out, sgn);
+        return;
     }
+    const uint32_t mask = (1u << (shift - 2)) - 1u, t = c >> (shift - 2);
+    const uint32_t x = 2 * (t >> (shift - 2)) + (lane >> 4), y = 4 * (t & mask) + ((lane >> 2) & 3),
+                   z = 4 * (c & mask) + (lane & 3);
+    const float d = eval<M>(s, coord(0, x), coord(1, y), coord(2, z));
+    CG_AT(out, ((size_t)x * n + y) * n + z, (uint64_t)n * n * n) = d;
     if (sgn) {
-        const uint32_t bits = __ballot_sync(0xFFFFFFFFu, pos) >> (lane & ~3u) & 0xFu;
+        const uint32_t b = __ballot_sync(0xFFFFFFFFu, (__float_as_uint(d) >> 31) == 0u);
+        const uint32_t bits = (b >> (lane & ~3u)) & 0xFu;
         if ((lane & 3) == 0 && bits)
             atomicOr(&CG_AT(sgn, (x * n + y) * W + (z >> 5), (uint64_t)n * n * W),
                      bits << (z & 31));
     }
 }
 
-// Large grids: each warp evaluates 2x4x4 bricks of corners (x, y, z), which
-// keeps the escape counts of a warp's lanes close (89% lane efficiency on the
-// 513^3 span vs 75% for 32 corners along z).  A work unit is a run of
-// `group` bricks along z.  With group 8 (grids with work for several waves)
-// the unit covers 32 consecutive distances of each of its 8 (x, y) rows
-// (whole 128-byte lines) and, with `sgn`, exactly one sign word per row:
-// one ballot per brick gives the signs, the z-lane-0 thread of each row
-// collects its row's 4 bits per brick and stores the finished word once (no
-// atomics; every word is written, padding bits 0).  With group 1 (smaller
-// grids, where 8-brick units would leave SMs idle) each brick's 4 bits go
-// into the word with atomicOr (sgn zeroed first).
+// Large grids: persistent warps take core units, then groups of 8 face items,
+// from `queue` (a unit of the bulb's inside costs seven of the outside, so a
+// fixed share left warps idle at the end: 309 against 285 us for the 257^3 span)
+// or, without one, in strides.  A warp asks for its next unit before it begins
+// the one it has.
+template <int M>
+__global__ void __launch_bounds__(256) k_de_grid_units(ShapeDev s, GridDev g,
+                                                       float* __restrict__ out,
+                                                       uint32_t* __restrict__ sgn, uint32_t W,
+                                                       uint32_t shift,
+                                                       uint32_t* __restrict__ queue,
+                                                       const GridDev* __restrict__ gp) {
+    if (gp) g = *gp;
+    const GridCoord coord{g};
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5, core = core_units(shift);
+    const uint32_t faces = face_items(shift), units = core + (faces + 7) / 8;
+    uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // the queue starts at nwarps
+    while (u < units) {
+        uint32_t next = u + nwarps;
+        if (queue && lane == 0) next = nwarps + atomicAdd(queue, 1u);
+        if (u < core) {
+            // y and z ranges turned by x: a warp's stride is a multiple of the
+            // words of a row, and it would else meet the same z range every
+            // time (the 513^3 span's mesh 3.03 against 2.9 ms).
+            const uint32_t a = shift - 5, b = shift - 2, x = u >> (a + b);
+            const uint32_t y = ((u >> a) + 37 * x) & ((1u << b) - 1u);
+            const uint32_t z = (u + x) & ((1u << a) - 1u);
+            core_unit<M>(s, coord, shift, W, (((x << b) | y) << a) | z, out, sgn);
+        } else {
+            const uint32_t f0 = 8 * (u - core), f1 = min(f0 + 8, faces);
+#pragma unroll 1
+            for (uint32_t f = f0; f < f1; ++f) face_item<M>(s, coord, shift, W, f, out, sgn);
+        }
+        u = queue ? __shfl_sync(0xFFFFFFFFu, next, 0) : next;
+    }
+}
+
+// Grids between: warps walk 2x4x4 bricks of corners (x, y, z), which keeps the
+// escape counts of a warp's lanes close (89% lane efficiency on the 513^3
+// span vs 75% for 32 corners along z); 8-brick units would leave SMs idle.
+// Each brick's 4 bits per row go into the sign word with atomicOr (sgn zeroed
+// first).
 template <int M>
 __global__ void __launch_bounds__(256) k_de_grid_brick(ShapeDev s, GridDev g,
                                                        float* __restrict__ out,
                                                        uint32_t* __restrict__ sgn, uint32_t W,
-                                                       uint32_t group,
                                                        const GridDev* __restrict__ gp) {
     if (gp) g = *gp;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t n = g.n;
-    const uint32_t BX = (n + 1) >> 1, BY = (n + 3) >> 2, BZ = (n + 3) >> 2;
-    const uint32_t GZ = (BZ + group - 1) / group;  // units along z
+    const uint32_t BX = (n + 1) >> 1, B4 = (n + 3) >> 2;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t dx = lane >> 4, dy = (lane >> 2) & 3, dz = lane & 3;
-    // Unit (bx, by, gz), advanced by the grid stride in the same mixed radix.
+    // Brick (bx, by, bz), advanced by the grid stride in the same mixed radix.
     const uint32_t u0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    uint32_t gz = u0 % GZ, by = (u0 / GZ) % BY, bx = u0 / (GZ * BY);
-    const uint32_t sz = nwarps % GZ, sy = (nwarps / GZ) % BY, sx = nwarps / (GZ * BY);
+    uint32_t bz = u0 % B4, by = (u0 / B4) % B4, bx = u0 / (B4 * B4);
+    const uint32_t sz = nwarps % B4, sy = (nwarps / B4) % B4, sx = nwarps / (B4 * B4);
     for (; bx < BX;) {
-        const uint32_t x = 2 * bx + dx, y = 4 * by + dy;
-        const bool row_ok = x < n && y < n;
-        const float px = grid_coord(g, 0, x), py = grid_coord(g, 1, y);
-        const uint32_t bz0 = gz * group, bz_end = min(bz0 + group, BZ);
-        uint32_t word = 0;
-        for (uint32_t bz = bz0; bz < bz_end; ++bz) {
-            const uint32_t z = 4 * bz + dz;
-            bool pos = false;
-            if (row_ok && z < n) {
-                const float d = eval<M>(s, px, py, grid_coord(g, 2, z));
-                CG_AT(out, ((size_t)x * n + y) * n + z, (uint64_t)n * n * n) = d;
-                pos = (__float_as_uint(d) >> 31) == 0u;
-            }
-            if (sgn) {
-                const uint32_t b = __ballot_sync(0xFFFFFFFFu, pos);
-                word |= ((b >> (lane & ~3u)) & 0xFu) << ((4 * bz) & 31);
-            }
+        const uint32_t x = 2 * bx + (lane >> 4), y = 4 * by + ((lane >> 2) & 3),
+                       z = 4 * bz + (lane & 3);
+        bool pos = false;
+        const bool in = x < n && y < n && z < n;
+        if (in) {
+            const float d =
+                eval<M>(s, grid_coord(g, 0, x), grid_coord(g, 1, y), grid_coord(g, 2, z));
+            CG_AT(out, ((size_t)x * n + y) * n + z, (uint64_t)n * n * n) = d;
+            pos = (__float_as_uint(d) >> 31) == 0u;
         }
-        if (sgn && dz == 0 && row_ok) {
-            uint32_t* wp = &CG_AT(sgn, (x * n + y) * W + ((4 * bz0) >> 5), (uint64_t)n * n * W);
-            if (group == 8) *wp = word;
-            else if (word) atomicOr(wp, word);
+        if (sgn) {
+            const uint32_t b = __ballot_sync(0xFFFFFFFFu, pos);
+            const uint32_t bits = (b >> (lane & ~3u)) & 0xFu;
+            if ((lane & 3) == 0 && bits)
+                atomicOr(&CG_AT(sgn, (x * n + y) * W + (z >> 5), (uint64_t)n * n * W),
+                         bits << (z & 31));
         }
-        gz += sz;
+        bz += sz;
         uint32_t carry = 0;
-        if (gz >= GZ) {
-            gz -= GZ;
+        if (bz >= B4) {
+            bz -= B4;
             carry = 1;
         }
         by += sy + carry;
         carry = 0;
-        if (by >= BY) {
-            by -= BY;
+        if (by >= B4) {
+            by -= B4;
             carry = 1;
         }
         bx += sx + carry;
@@ -425,9 +456,11 @@ static void launch_grid_mode(const ShapeDev& s, const GridDev& g, float* out, ui
     // grid in more waves than k_de_grid_small's 44, and one corner per thread
     // in row order keeps 24 lanes busy against 27 (15.8 against 14.7 us).
     if (k == DE_GRID_AUTO) k = g.n > 65 ? DE_GRID_BRICK : DE_GRID_LINEAR;
-    if (g_de_grid_kernel == DE_GRID_AUTO && k == DE_GRID_LINEAR) {
-        const uint64_t b4 = (g.n + 3) >> 2, bricks = ((g.n + 1) >> 1) * b4 * b4;
-        k_de_grid_small<M><<<(unsigned)((bricks + 3) / 4), 128, 0, st>>>(s, g, out, sgn, W, gp);
+    uint32_t shift = 0;
+    while ((2u << shift) < g.n) ++shift;
+    if (g_de_grid_kernel == DE_GRID_AUTO && k == DE_GRID_LINEAR && g.n > kUnitMinRes) {
+        const uint32_t warps = core_bricks(shift) + face_items(shift);
+        k_de_grid_small<M><<<(warps + 3) / 4, 128, 0, st>>>(s, g, out, sgn, W, shift, gp);
     } else if (k == DE_GRID_PACKED && (M == MODE_P8 || M == MODE_P8_IT15)) {
         const uint64_t b4 = (g.n + 3) >> 2;
         k_de_grid_p8x2<<<grid_for(b4 * b4 * b4 * 32, B, 8), B, 0, st>>>(s, g, out, sgn, W, gp);
@@ -437,9 +470,14 @@ static void launch_grid_mode(const ShapeDev& s, const GridDev& g, float* out, ui
         const uint64_t rows = (uint64_t)((g.n + 1) >> 1) * ((g.n + 3) >> 2);
         const uint64_t bz = (g.n + 3) >> 2;
         const uint64_t units8 = rows * ((bz + 7) / 8);
-        const uint32_t group = units8 >= 4ull * sm_count() * 8 * (B / 32) ? 8u : 1u;
-        const uint64_t units = rows * ((bz + group - 1) / group);
-        k_de_grid_brick<M><<<grid_for(units * 32, B, 8), B, 0, st>>>(s, g, out, sgn, W, group, gp);
+        if (units8 >= 4ull * sm_count() * 8 * (B / 32)) {
+            const uint64_t units = core_units(shift) + (face_items(shift) + 7) / 8;
+            uint32_t* queue = sgn ? sgn + (size_t)g.n * g.n * W : nullptr;
+            k_de_grid_units<M><<<grid_for(units * 32, B, 8), B, 0, st>>>(
+                s, g, out, sgn, W, shift, queue, gp);
+        } else {
+            k_de_grid_brick<M><<<grid_for(rows * bz * 32, B, 8), B, 0, st>>>(s, g, out, sgn, W, gp);
+        }
     } else {
         const uint64_t total = (uint64_t)g.n * g.n * g.n;
         k_de_grid<M><<<grid_for(total, B, 8), B, 0, st>>>(s, g, out, sgn, W, gp);

@@ -46,8 +46,9 @@ int set_de_grid_kernel(int v);
 int de_grid_kernel_option();
 uint32_t place_blocks_per_sm();
 
-// Step 1 on a span grid.  With `sgn` (zeroed, (res+1)^2 rows x W words) the
-// kernel also packs is_sign_positive of every corner into sign words.
+// Step 1 on a span grid.  With `sgn` (zeroed, (res+1)^2 rows x W words, and one
+// word more for a work queue) the kernel also packs is_sign_positive of every
+// corner into sign words.
 // With `gp` the kernels take the grid from device memory instead of `g`
 // (which still fixes the launch shape): a captured graph then serves every
 // span of the same resolution.
@@ -84,7 +85,7 @@ enum : uint32_t { MESH_LERP_FAIL = 1u };
 // Device workspace of one span mesh (sizes from mesh_workspace_layout).
 struct MeshWork {
     float* dists;        // (res+1)^3 corner distances
-    uint32_t* sgn;       // sign words: (res+1)^2 rows x W words
+    uint32_t* sgn;       // sign words: (res+1)^2 rows x W words, then step 1's queue
     uint32_t* cellbits;  // surface-cell words: res^2 rows x Wc words
     uint32_t* wordoff;   // vertices before each cell word, within its row
     uint32_t* rowcnt;    // vertices per cell row

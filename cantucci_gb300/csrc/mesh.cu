@@ -42,7 +42,7 @@ size_t mesh_workspace_layout(uint32_t res, char* base, MeshWork* w) {
     };
     MeshWork t;
     t.dists = (float*)take(n3 * 4);
-    t.sgn = (uint32_t*)take(rows_c * d.W * 4);
+    t.sgn = (uint32_t*)take((rows_c * d.W + 1) * 4);  // and step 1's queue
     t.cellbits = (uint32_t*)take(rows * d.Wc * 4);
     t.wordoff = (uint32_t*)take(rows * d.Wc * 4);
     t.rowcnt = (uint32_t*)take(rows * 4);

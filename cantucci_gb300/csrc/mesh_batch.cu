@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "grid_units.cuh"
 #include "kernels.cuh"
 #include "mesh_rows.cuh"
 
@@ -48,7 +49,9 @@ struct BatchJob {
     uint32_t row_begin;         // first global cell row
     uint32_t item_begin;        // first global step-1 work item
     uint32_t items;
-    uint32_t brick;             // 1: runs of 8 2x4x4 bricks along z, 0: 32 consecutive corners
+    // 2: core units and groups of 8 face items (grid_units.cuh), 1: runs of 8
+    // 2x4x4 bricks along z (res < 32), 0: 32 consecutive corners
+    uint32_t brick;
 };
 
 struct BatchTotals {
@@ -97,6 +100,13 @@ __device__ __forceinline__ float job_coord(const BatchJob& j, int k, uint32_t v)
     return __fadd_rn(j.start[k], __fmul_rn(j.across[k], __fmul_rn((float)v, j.inv_res)));
 }
 
+struct JobCoord {
+    const BatchJob& j;
+    __device__ __forceinline__ float operator()(int k, uint32_t v) const {
+        return job_coord(j, k, v);
+    }
+};
+
 // Step 1 over all spans: persistent warps pull chunks of items from `queue`.
 template <int M>
 __global__ void k_batch_de(ShapeDev s, const BatchJob* __restrict__ jobs, uint32_t njobs,
@@ -117,9 +127,20 @@ __global__ void k_batch_de(ShapeDev s, const BatchJob* __restrict__ jobs, uint32
             float* out = dists + J.dist_off;
             uint32_t* sg = sgn + J.sgn_off;
             const uint32_t local = item - J.item_begin;
-            if (J.brick) {
-                // Unit (bx, by, gz): the 8 bricks along z of sign word gz, as
-                // k_de_grid_brick walks them; the word is stored whole.
+            if (J.brick == 2) {
+                const JobCoord coord{J};
+                const uint32_t shift = J.d.shift, core = core_units(shift);
+                if (local < core) {
+                    core_unit<M>(s, coord, shift, W, local, out, sg);
+                } else {
+                    const uint32_t f0 = 8 * (local - core), f1 = min(f0 + 8, face_items(shift));
+#pragma unroll 1
+                    for (uint32_t f = f0; f < f1; ++f)
+                        face_item<M>(s, coord, shift, W, f, out, sg);
+                }
+            } else if (J.brick) {
+                // Unit (bx, by, gz): the 8 bricks along z of sign word gz; the
+                // word is stored whole.
                 const uint32_t BY = (n + 3) >> 2, BZ = (n + 3) >> 2;
                 const uint32_t gz = local % W, t = local / W, by = t % BY, bx = t / BY;
                 const uint32_t dx = lane >> 4, dy = (lane >> 2) & 3, dz = lane & 3;
@@ -307,9 +328,10 @@ cg_status plan_items(std::vector<BatchJob>& jobs, uint32_t brick_min_res, uint32
     uint64_t items = 0;
     for (BatchJob& J : jobs) {
         const uint64_t n = J.d.n;
-        J.brick = J.d.res >= brick_min_res ? 1u : 0u;
-        J.items = J.brick ? (uint32_t)(((n + 1) >> 1) * ((n + 3) >> 2) * J.d.W)
-                          : (uint32_t)((n * n * n + 31) / 32);
+        J.brick = J.d.res < brick_min_res ? 0u : (J.d.res < kUnitMinRes ? 1u : 2u);
+        J.items = J.brick == 2   ? core_units(J.d.shift) + (face_items(J.d.shift) + 7) / 8
+                  : J.brick == 1 ? (uint32_t)(((n + 1) >> 1) * ((n + 3) >> 2) * J.d.W)
+                                 : (uint32_t)((n * n * n + 31) / 32);
         J.item_begin = (uint32_t)items;
         items += J.items;
         if (items > 0x7FFFFFFFull) {
