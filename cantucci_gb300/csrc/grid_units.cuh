@@ -58,39 +58,57 @@ __device__ __forceinline__ void core_unit(const ShapeDev& s, const Coord& coord,
     if (sgn && (lane & 3) == 0) CG_AT(sgn, row * W + gz, (uint64_t)n * n * W) = word;
 }
 
+// Lane `lane`'s corner of face item f; `row_word`: the item is one sign word of
+// a row, else part of the plane z = res.
+struct FaceCorner {
+    uint32_t x, y, z;
+    bool in, row_word;
+};
+
+__device__ __forceinline__ FaceCorner face_corner(uint32_t shift, uint32_t f, uint32_t lane) {
+    const uint32_t res = 1u << shift, n = res + 1u, rows = face_row_items(shift);
+    FaceCorner c;
+    c.row_word = f < rows;
+    if (c.row_word) {
+        const uint32_t r = f >> (shift - 5);
+        c.x = r <= res ? res : r - n;
+        c.y = r <= res ? r : res;
+        c.z = 32 * (f & ((1u << (shift - 5)) - 1u)) + lane;
+        c.in = true;
+    } else {
+        const uint32_t i = (f - rows) * 32 + lane;
+        c.in = i < n * n;
+        c.x = i / n;
+        c.y = i - c.x * n;
+        c.z = res;
+    }
+    return c;
+}
+
+// The item's signs from its ballot: a row's word whole, or the first bit of
+// each row's last word (its only corner).
+__device__ __forceinline__ void face_sign(const FaceCorner& c, uint32_t W, uint32_t ballot,
+                                          bool pos, uint32_t lane, uint32_t n,
+                                          uint32_t* __restrict__ sgn) {
+    if (c.row_word ? lane == 0 : c.in)
+        CG_AT(sgn, (c.x * n + c.y) * W + (c.z >> 5), (uint64_t)n * n * W) =
+            c.row_word ? ballot : (pos ? 1u : 0u);
+}
+
 template <int M, class Coord>
 __device__ __forceinline__ void face_item(const ShapeDev& s, const Coord& coord, uint32_t shift,
                                           uint32_t W, uint32_t f, float* __restrict__ out,
                                           uint32_t* __restrict__ sgn) {
-    const uint32_t lane = threadIdx.x & 31, res = 1u << shift, n = res + 1u;
-    const uint32_t rows = face_row_items(shift);
-    uint32_t x, y, z;
-    bool in = true;
-    if (f < rows) {
-        const uint32_t r = f >> (shift - 5);
-        x = r <= res ? res : r - n;
-        y = r <= res ? r : res;
-        z = 32 * (f & ((1u << (shift - 5)) - 1u)) + lane;
-    } else {
-        const uint32_t i = (f - rows) * 32 + lane;
-        in = i < n * n;
-        x = i / n;
-        y = i - x * n;
-        z = res;
-    }
+    const uint32_t lane = threadIdx.x & 31, n = (1u << shift) + 1u;
+    const FaceCorner c = face_corner(shift, f, lane);
     bool pos = false;
-    if (in) {
-        const float d = eval<M>(s, coord(0, x), coord(1, y), coord(2, z));
-        CG_AT(out, ((size_t)x * n + y) * n + z, (uint64_t)n * n * n) = d;
+    if (c.in) {
+        const float d = eval<M>(s, coord(0, c.x), coord(1, c.y), coord(2, c.z));
+        CG_AT(out, ((size_t)c.x * n + c.y) * n + c.z, (uint64_t)n * n * n) = d;
         pos = (__float_as_uint(d) >> 31) == 0u;
     }
     if (!sgn) return;
-    const uint32_t bits = __ballot_sync(0xFFFFFFFFu, pos);
-    if (f < rows) {
-        if (lane == 0) CG_AT(sgn, (x * n + y) * W + (z >> 5), (uint64_t)n * n * W) = bits;
-    } else if (in) {
-        CG_AT(sgn, (x * n + y) * W + (res >> 5), (uint64_t)n * n * W) = pos ? 1u : 0u;
-    }
+    face_sign(c, W, __ballot_sync(0xFFFFFFFFu, pos), pos, lane, n, sgn);
 }
 
 }  // namespace cg

@@ -508,7 +508,7 @@ __global__ void __launch_bounds__(256) k_quad_emit_fine(const uint32_t* __restri
         const uint32_t below = bit - 1u;
         q += __popc(e.ex & below) + __popc(e.ey & below) + __popc(e.ez & below);
         const EdgeWords mine = {e.ex & bit, e.ey & bit, e.ez & bit};
-        quad_emit_word(mine, d, dists, cellbits, wordoff, rowoff, 0u, q, idx, icap, x, y, w);
+        quad_emit_word(mine, d, sgn, dists, cellbits, wordoff, rowoff, 0u, q, idx, icap, x, y, w);
     }
 }
 

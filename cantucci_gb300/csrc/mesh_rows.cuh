@@ -471,11 +471,40 @@ __device__ __forceinline__ uint32_t vertex_id(const MeshDims& d, const uint32_t*
            __popc(CG_AT(cellbits, r * d.Wc + w, nc) & ((1u << b) - 1u));
 }
 
+// The two triangles of a quad with corners v0, v1, v2, v3 (buffer.rs:288-372):
+// (v0 v1 v2)(v1 v3 v2), or with `flip` (v0 v2 v1)(v1 v2 v3).  `pairs`: idx is
+// 8-byte aligned.
+__device__ __forceinline__ void quad_store(uint32_t* __restrict__ idx, uint64_t icap, bool pairs,
+                                           uint64_t q, bool flip, uint32_t v0, uint32_t v1,
+                                           uint32_t v2, uint32_t v3) {
+    if (6 * q + 6 > icap) return;
+    const uint32_t b = flip ? v2 : v1, c = flip ? v1 : v2;  // v0 b c, v1 then
+    const uint32_t e = flip ? v2 : v3, f = flip ? v3 : v2;  // v1 e f
+#ifndef CG_CHECKED
+    if (pairs) {
+        uint2* o = reinterpret_cast<uint2*>(idx) + 3 * q;
+        o[0] = make_uint2(v0, b);
+        o[1] = make_uint2(c, v1);
+        o[2] = make_uint2(e, f);
+        return;
+    }
+#endif
+    const uint32_t t[6] = {v0, b, c, v1, e, f};
+#pragma unroll
+    for (int k = 0; k < 6; ++k) CG_AT(idx, 6 * q + k, icap) = t[k];
+}
+
 // Quad indices of corner row (x, y), sign word w (buffer.rs:288-372), from
 // quad q on: corner order, then +x, +y, +z; winding by dists[(x, y, z)] <
 // 0.0.  Vertex ids are rowoff-based minus `vbase`; quad q is written from
 // index 6 * q (capacity icap).  Returns the next quad.
+//
+// The four cell rows around the corner row give all the word's vertex ids: of
+// row k, p_k = the cells before z is the id of cell z, and p_k - 1 that of
+// cell z - 1 (a quad's cells are surface cells), also across a word boundary.
+// Twelve loads to a word instead of twelve to a quad.
 __device__ __forceinline__ uint64_t quad_emit_word(const EdgeWords& e, const MeshDims& d,
+                                                   const uint32_t* __restrict__ sgn,
                                                    const float* __restrict__ dists,
                                                    const uint32_t* __restrict__ cellbits,
                                                    const uint32_t* __restrict__ wordoff,
@@ -484,46 +513,35 @@ __device__ __forceinline__ uint64_t quad_emit_word(const EdgeWords& e, const Mes
                                                    uint32_t* __restrict__ idx, uint64_t icap,
                                                    uint32_t x, uint32_t y, uint32_t w) {
     uint32_t any = e.ex | e.ey | e.ez;
+    if (!any) return q;
+    const bool pairs = (reinterpret_cast<uintptr_t>(idx) & 7u) == 0u;
+    [[maybe_unused]] const uint64_t nr = (uint64_t)d.res * d.res, nc = nr * d.Wc;
+    // Rows (x, y), (x, y-1), (x-1, y), (x-1, y-1); those off the grid take no
+    // part in a quad.
+    uint32_t base[4], bits[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        base[k] = bits[k] = 0;
+        if ((k & 1) > y || ((k >> 1) & 1) > x) continue;
+        const uint32_t r = ((x - (k >> 1)) << d.shift) + y - (k & 1);
+        base[k] = CG_AT(rowoff, r, nr) + CG_AT(wordoff, r * d.Wc + w, nc) - vbase;
+        bits[k] = CG_AT(cellbits, r * d.Wc + w, nc);
+    }
+    const size_t corner = ((size_t)x * d.n + y) * d.n + w * 32;
+    const uint32_t positive =
+        CG_AT(sgn, (x * d.n + y) * d.W + w, (uint64_t)d.n * d.n * d.W);
     while (any) {
-        const uint32_t b = __ffs(any) - 1;
+        const uint32_t b = __ffs(any) - 1, bit = 1u << b;
         any &= any - 1;
-        const uint32_t z = w * 32 + b;
-        const bool neg = CG_AT(dists, ((size_t)x * d.n + y) * d.n + z, (uint64_t)d.n * d.n * d.n) < 0.0f;
-        const uint32_t bit = 1u << b;
-        uint32_t t[6];
-        if (e.ex & bit) {
-            const uint32_t v0 = vertex_id(d, cellbits, wordoff, rowoff, x, y - 1, z - 1) - vbase;
-            const uint32_t v1 = vertex_id(d, cellbits, wordoff, rowoff, x, y - 1, z) - vbase;
-            const uint32_t v2 = vertex_id(d, cellbits, wordoff, rowoff, x, y, z - 1) - vbase;
-            const uint32_t v3 = vertex_id(d, cellbits, wordoff, rowoff, x, y, z) - vbase;
-            if (neg) { t[0] = v0; t[1] = v2; t[2] = v1; t[3] = v1; t[4] = v2; t[5] = v3; }
-            else     { t[0] = v0; t[1] = v1; t[2] = v2; t[3] = v1; t[4] = v3; t[5] = v2; }
-            if (6 * q + 6 <= icap)
-                for (int k = 0; k < 6; ++k) CG_AT(idx, 6 * q + k, icap) = t[k];
-            ++q;
-        }
-        if (e.ey & bit) {
-            const uint32_t v0 = vertex_id(d, cellbits, wordoff, rowoff, x - 1, y, z - 1) - vbase;
-            const uint32_t v1 = vertex_id(d, cellbits, wordoff, rowoff, x - 1, y, z) - vbase;
-            const uint32_t v2 = vertex_id(d, cellbits, wordoff, rowoff, x, y, z - 1) - vbase;
-            const uint32_t v3 = vertex_id(d, cellbits, wordoff, rowoff, x, y, z) - vbase;
-            if (neg) { t[0] = v0; t[1] = v1; t[2] = v2; t[3] = v1; t[4] = v3; t[5] = v2; }
-            else     { t[0] = v0; t[1] = v2; t[2] = v1; t[3] = v1; t[4] = v2; t[5] = v3; }
-            if (6 * q + 6 <= icap)
-                for (int k = 0; k < 6; ++k) CG_AT(idx, 6 * q + k, icap) = t[k];
-            ++q;
-        }
-        if (e.ez & bit) {
-            const uint32_t v0 = vertex_id(d, cellbits, wordoff, rowoff, x - 1, y - 1, z) - vbase;
-            const uint32_t v1 = vertex_id(d, cellbits, wordoff, rowoff, x - 1, y, z) - vbase;
-            const uint32_t v2 = vertex_id(d, cellbits, wordoff, rowoff, x, y - 1, z) - vbase;
-            const uint32_t v3 = vertex_id(d, cellbits, wordoff, rowoff, x, y, z) - vbase;
-            if (neg) { t[0] = v0; t[1] = v2; t[2] = v1; t[3] = v1; t[4] = v2; t[5] = v3; }
-            else     { t[0] = v0; t[1] = v1; t[2] = v2; t[3] = v1; t[4] = v3; t[5] = v2; }
-            if (6 * q + 6 <= icap)
-                for (int k = 0; k < 6; ++k) CG_AT(idx, 6 * q + k, icap) = t[k];
-            ++q;
-        }
+        // (a negative sign bit is also that of -0 and NaN, which are not < 0)
+        const bool neg = !(positive & bit) &&
+                         CG_AT(dists, corner + b, (uint64_t)d.n * d.n * d.n) < 0.0f;
+        uint32_t p[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) p[k] = base[k] + __popc(bits[k] & (bit - 1u));
+        if (e.ex & bit) quad_store(idx, icap, pairs, q++, neg, p[1] - 1, p[1], p[0] - 1, p[0]);
+        if (e.ey & bit) quad_store(idx, icap, pairs, q++, !neg, p[2] - 1, p[2], p[0] - 1, p[0]);
+        if (e.ez & bit) quad_store(idx, icap, pairs, q++, neg, p[3], p[2], p[1], p[0]);
     }
     return q;
 }
@@ -538,7 +556,7 @@ __device__ __forceinline__ void quad_emit_row(const uint32_t* __restrict__ sgn, 
                                               uint32_t r) {
     const uint32_t x = r >> d.shift, y = r & (d.res - 1);
     for (uint32_t w = 0; w < d.Wc; ++w)
-        q = quad_emit_word(edge_words(sgn, d, x, y, w), d, dists, cellbits, wordoff, rowoff, vbase,
+        q = quad_emit_word(edge_words(sgn, d, x, y, w), d, sgn, dists, cellbits, wordoff, rowoff, vbase,
                            q, idx, icap, x, y, w);
 }
 
