@@ -143,6 +143,7 @@ SIGNATURES = [
     ("cg_de_grad_tangent", _i32, [_shp, _vp, _u64, _u32, _vp, _vp]),
     ("cg_de_spatial_grad", _i32, [_shp, _vp, _u64, _vp, _vp]),
     ("cg_de_backward", _i32, [_shp, _vp, _vp, _u64, _vp, _vp, _vp]),
+    ("cg_surface_l1", _i32, [_shp, _vp, _u64, _f32, _vp, _vp]),
     ("cg_fd_grad", _i32, [_shp, _vp, _u64, _f32, _vp, _vp]),
     ("cg_set_option", _i32, [C.c_char_p, C.c_int64]),
     ("cg_mesher_stream", _i32, [_vp, C.POINTER(_vp)]),

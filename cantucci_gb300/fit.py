@@ -173,25 +173,23 @@ def _make_surface_fn():
 
     class SurfaceL1(torch.autograd.Function):
         """mean |DE(p_i; power, rot)| and its gradient from one adjoint pass
-        per point (cg_de_grad), without the points whose |dDE/dtheta_k|
+        per point (cg_surface_l1), without the points whose |dDE/dtheta_k|
         exceeds cap."""
 
         @staticmethod
         def forward(ctx, power, rot, points, max_iters, bailout, cap):
-            from .autograd import de_grad
-            g = de_grad(points, float(power), [float(v) for v in rot.detach().cpu()], max_iters,
-                        bailout)
-            ok = torch.isfinite(g).all(dim=1)
-            n = ok.sum().clamp(min=1)
-            de = g[:, 0]
-            loss = de[ok].abs().sum() / n
-            J = g[:, 4:8]
-            keep = ok & (J.abs().max(dim=1).values <= cap) if cap > 0 else ok
-            grad = (torch.sign(de[keep])[:, None] * J[keep]).sum(dim=0) / n
-            ctx.save_for_backward(grad)
+            pts = points.contiguous().float()
+            out = torch.empty(5, dtype=torch.float32, device=pts.device)
+            shape = _shape(float(power), [float(v) for v in rot.detach().cpu()], max_iters,
+                           bailout)
+            check(load().cg_surface_l1(
+                C.byref(shape), C.c_void_p(pts.data_ptr()), pts.shape[0], max(float(cap), 0.0),
+                C.c_void_p(out.data_ptr()),
+                C.c_void_p(torch.cuda.current_stream(pts.device).cuda_stream)))
+            ctx.save_for_backward(out[1:])
             ctx.devs = (power.device if torch.is_tensor(power) else None,
                         rot.device if torch.is_tensor(rot) else None)
-            return loss
+            return out[0].clone()
 
         @staticmethod
         def backward(ctx, gout):

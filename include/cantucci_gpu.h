@@ -520,6 +520,14 @@ cg_status cg_de_spatial_grad(const cg_shape* shape, const float* points, uint64_
 cg_status cg_de_backward(const cg_shape* shape, const float* points, const float* grad_out,
                          uint64_t n, float* grad_points, float* grad_params, void* stream);
 
+/* Mean |DE| over the points (device, n x 3) whose DE and derivatives are all
+ * finite, and its gradient with respect to (power, a, b, c) without the points
+ * of which some |dDE/dtheta_k| exceeds cap (0: none), divided by the same
+ * number of points.  out: device, 5 floats (0 for no points).  Sums in double,
+ * in a fixed order; the calling thread's scratch buffer as cg_de_backward. */
+cg_status cg_surface_l1(const cg_shape* shape, const float* points, uint64_t n, float cap,
+                        float* out, void* stream);
+
 /* Central-difference gradient with six estimator calls per point and step h
  * (the normal of src/mesh/buffer.rs:256-266, scaled by 1/2h), any shape.
  * out: device, n x 3 floats. */
