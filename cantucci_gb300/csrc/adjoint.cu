@@ -98,16 +98,17 @@ __global__ void __launch_bounds__(128) k_de_spatial_grad(ShapeDev s, const float
 }
 
 // Vector-Jacobian product of a batch: g[i] * dDE/dp into grad_points (n x 3)
-// and, per warp, the sum over its points of g[i] * dDE/d(power, euler) into
-// partial[4 w .. 4 w + 3] (added up by k_sum_partials4 in a fixed order, so
-// the result does not depend on scheduling).
+// and, per warp, the sum over its points of g[i] * dDE/d(power, euler), in
+// double, into partial[4 w .. 4 w + 3] (added up by k_sum_partials4 in a fixed
+// order, so the result does not depend on scheduling; the terms of chaotic
+// points cancel over ten decades).
 template <bool LONG>
 __global__ void __launch_bounds__(128) k_de_vjp(ShapeDev s, Dm3 dm, const float* __restrict__ pts,
                                                 const float* __restrict__ g, uint64_t n,
-                                                float* __restrict__ gp, float* __restrict__ params) {
+                                                float* __restrict__ gp, double* __restrict__ params) {
     extern __shared__ __align__(16) float4 adj_smem[];
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         float o[8];
         const float x = pts[3 * i], y = pts[3 * i + 1], z = pts[3 * i + 2];
@@ -133,40 +134,30 @@ __global__ void __launch_bounds__(128) k_de_vjp(ShapeDev s, Dm3 dm, const float*
         const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            float v = acc[k];
+            double v = acc[k];
             for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, o);
             if ((threadIdx.x & 31) == 0) params[4 * w + k] = v;
         }
     }
 }
 
-// params[k] += the sum over warps w < nwarps of partial[4 w + k], in a fixed
-// order (one block: strided sequential sums of one 16-byte load per warp,
-// then a fixed tree).  `partial` is 16-byte aligned.
-__global__ void __launch_bounds__(256) k_sum_partials4(const float* __restrict__ partial,
-                                                       uint32_t nwarps, float* __restrict__ params) {
-    __shared__ float sh[4][256];
-    const float4* p4 = reinterpret_cast<const float4*>(partial);
-    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    for (uint32_t w = threadIdx.x; w < nwarps; w += 256) {
-        const float4 q = p4[w];
-        v.x += q.x;
-        v.y += q.y;
-        v.z += q.z;
-        v.w += q.w;
-    }
-    sh[0][threadIdx.x] = v.x;
-    sh[1][threadIdx.x] = v.y;
-    sh[2][threadIdx.x] = v.z;
-    sh[3][threadIdx.x] = v.w;
+// params[k] = the sum over warps w < nwarps of partial[4 w + k], in a fixed
+// order: strided sequential sums, eight warps to a column, then a fixed tree.
+__global__ void __launch_bounds__(1024) k_sum_partials4(const double* __restrict__ partial,
+                                                        uint32_t nwarps,
+                                                        float* __restrict__ params) {
+    __shared__ double sh[32];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = warp & 3;
+    double v = 0.0;
+    for (uint32_t w = (warp >> 2) * 32 + lane; w < nwarps; w += 256) v += partial[4 * w + k];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, o);
+    if (lane == 0) sh[warp] = v;
     __syncthreads();
-    for (uint32_t half = 128; half > 0; half >>= 1) {
-        if (threadIdx.x < half)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) sh[k][threadIdx.x] += sh[k][threadIdx.x + half];
-        __syncthreads();
+    if (threadIdx.x < 4) {
+        double t = 0.0;
+        for (int i = 0; i < 8; ++i) t += sh[4 * i + threadIdx.x];
+        params[threadIdx.x] = (float)t;
     }
-    if (threadIdx.x < 4) params[threadIdx.x] += sh[threadIdx.x][0];
 }
 
 // Mean |DE| over the points whose DE and derivatives are all finite, and its
@@ -292,7 +283,7 @@ cg_status release_partials(float* partial, cudaStream_t st) {
 
 cg_status launch_sum_partials4(const float* partial, uint32_t nwarps, float* params,
                                cudaStream_t st) {
-    k_sum_partials4<<<1, 256, 0, st>>>(partial, nwarps, params);
+    k_sum_partials4<<<1, 1024, 0, st>>>(reinterpret_cast<const double*>(partial), nwarps, params);
     CG_CHECK_LAUNCH("k_sum_partials4");
     return CG_OK;
 }
@@ -484,8 +475,10 @@ cg_status cg_de_backward(const cg_shape* shape, const float* points, const float
         return CG_EINVAL;
     }
     cudaStream_t st = (cudaStream_t)stream;
-    if (grad_params) CG_CUDA(cudaMemsetAsync(grad_params, 0, 4 * sizeof(float), st));
-    if (!n) return CG_OK;
+    if (!n) {
+        if (grad_params) CG_CUDA(cudaMemsetAsync(grad_params, 0, 4 * sizeof(float), st));
+        return CG_OK;
+    }
     const bool lng = shape->max_iters <= ADJ_LONG_MAX;
     const unsigned B = lng ? ADJ_LONG_BLOCK : ADJ_BLOCK;
     const size_t smem = lng ? long_tape_bytes(shape->max_iters, B)
@@ -495,9 +488,9 @@ cg_status cg_de_backward(const cg_shape* shape, const float* points, const float
     CG_TRY(adj_launch_shape(kernel, B, smem, n, &G));
     const uint32_t nwarps = G * (B / 32);
     float* partial = nullptr;
-    if (grad_params) CG_TRY(acquire_partials((size_t)nwarps * 4, st, &partial));
+    if (grad_params) CG_TRY(acquire_partials((size_t)nwarps * 8, st, &partial));
     kernel<<<G, B, smem, st>>>(make_shape_dev(*shape), rotation_derivatives(*shape), points,
-                               grad_out, n, grad_points, partial);
+                               grad_out, n, grad_points, reinterpret_cast<double*>(partial));
     cg_status rs = cuda_status(cudaGetLastError(), "k_de_vjp", __FILE__, __LINE__);
     if (rs == CG_OK && partial) rs = launch_sum_partials4(partial, nwarps, grad_params, st);
     if (partial) {

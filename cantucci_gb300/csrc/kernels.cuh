@@ -177,8 +177,8 @@ cg_status launch_points_table(const MeshDims& d, const MeshWork& w, uint32_t* po
 cg_status launch_exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* scratch,
                                 uint32_t* total, cudaStream_t st);
 size_t scan_scratch_words(uint32_t n);
-// params[k] += the sum over nwarps per-warp partials partial[4 w + k], in a
-// fixed order (deterministic parameter gradients).
+// params[k] = the sum over nwarps per-warp partials, doubles [4 w + k] at
+// `partial`, in a fixed order (deterministic parameter gradients).
 cg_status launch_sum_partials4(const float* partial, uint32_t nwarps, float* params,
                                cudaStream_t st);
 // The calling thread's scratch buffer (at least `floats` words, 16-byte

@@ -216,10 +216,10 @@ template <bool LONG>
 __global__ void __launch_bounds__(128) k_trace_backward(ShapeDev s, CameraDev c, Dm3 dm,
                                                         const float* __restrict__ depth,
                                                         const float* __restrict__ g, float cap,
-                                                        float* __restrict__ params) {
+                                                        double* __restrict__ params) {
     extern __shared__ __align__(16) float4 adj_smem[];
     const uint32_t n = c.width * c.height;
-    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float t = depth[i], gi = g[i];
         if (!(t > 0.0f) || gi == 0.0f) continue;
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(128) k_trace_backward(ShapeDev s, CameraDev c,
     const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        float v = acc[k];
+        double v = acc[k];
         for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, off);
         if ((threadIdx.x & 31) == 0) params[4 * w + k] = v;
     }
@@ -423,7 +423,6 @@ cg_status cg_trace_backward_capped(const cg_shape* shape, const cg_camera* camer
     const CameraDev c = make_camera(*camera);
     const Dm3 dm = rotation_derivatives(*shape);
     cudaStream_t st = (cudaStream_t)stream;
-    CG_CUDA(cudaMemsetAsync(grad_params, 0, 4 * sizeof(float), st));
     const uint64_t n = (uint64_t)c.width * c.height;
     const bool lng = shape->max_iters <= ADJ_LONG_MAX;
     const unsigned B = lng ? ADJ_LONG_BLOCK : ADJ_BLOCK;
@@ -434,8 +433,9 @@ cg_status cg_trace_backward_capped(const cg_shape* shape, const cg_camera* camer
     CG_TRY(adj_launch_shape(kernel, B, smem, n, &G));
     const uint32_t nwarps = G * (B / 32);
     float* partial = nullptr;
-    CG_TRY(acquire_partials((size_t)nwarps * 4, st, &partial));
-    kernel<<<G, B, smem, st>>>(s, c, dm, depth, grad_depth, cap, partial);
+    CG_TRY(acquire_partials((size_t)nwarps * 8, st, &partial));
+    kernel<<<G, B, smem, st>>>(s, c, dm, depth, grad_depth, cap,
+                               reinterpret_cast<double*>(partial));
     cg_status rs = cuda_status(cudaGetLastError(), "k_trace_backward", __FILE__, __LINE__);
     if (rs == CG_OK) rs = launch_sum_partials4(partial, nwarps, grad_params, st);
     const cg_status rr = release_partials(partial, st);
