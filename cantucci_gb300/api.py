@@ -9,6 +9,7 @@ Where the reference panics, these raise CantucciError (or AssertionError for
 the constructor asserts).  Device arrays are torch CUDA tensors; host arrays
 are numpy.  All compute runs in libcantucci_gpu.so; there is no CPU path.
 """
+import contextlib
 import ctypes as C
 import threading
 
@@ -29,6 +30,27 @@ def _torch():
 def _stream_ptr(device=None):
     torch = _torch()
     return C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+
+
+def _device_points(torch, points):
+    """(whether `points` is a CUDA tensor, it as contiguous (n, 3) float32 on
+    a GPU).  The tensor that is all that already is taken as it is: the calls
+    below cost more than the kernel on a small batch."""
+    on_dev = isinstance(points, torch.Tensor) and points.is_cuda
+    if (on_dev and points.dtype == torch.float32 and points.dim() == 2 and points.shape[1] == 3
+            and points.is_contiguous()):
+        return True, points
+    pts = points if on_dev else torch.as_tensor(np.ascontiguousarray(points, np.float32))
+    return on_dev, pts.reshape(-1, 3).to(device="cuda" if not on_dev else pts.device,
+                                         dtype=torch.float32).contiguous()
+
+
+_HERE = contextlib.nullcontext()
+
+
+def _on_device(torch, device):
+    """Makes `device` current, which most often it is."""
+    return _HERE if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 class Span:
@@ -88,16 +110,12 @@ class Shape:
         `points` is an (n, 3) float32 CUDA tensor (result: CUDA tensor) or a
         host array (result: numpy array)."""
         torch = _torch()
-        lib = load()
-        on_dev = isinstance(points, torch.Tensor) and points.is_cuda
-        pts = points if on_dev else torch.as_tensor(np.ascontiguousarray(points, np.float32))
-        pts = pts.reshape(-1, 3).to(device="cuda" if not on_dev else pts.device,
-                                    dtype=torch.float32).contiguous()
+        on_dev, pts = _device_points(torch, points)
         out = torch.empty(pts.shape[0], dtype=torch.float32, device=pts.device)
-        with torch.cuda.device(pts.device):
-            check(lib.cg_min_distance_from(C.byref(self._cshape()), C.c_void_p(pts.data_ptr()),
-                                           pts.shape[0], C.c_void_p(out.data_ptr()),
-                                           self.numerics, _stream_ptr(pts.device)))
+        with _on_device(torch, pts.device):
+            check(load().cg_min_distance_from(C.byref(self._cshape()), pts.data_ptr(),
+                                              pts.shape[0], out.data_ptr(), self.numerics,
+                                              _stream_ptr(pts.device)))
         return out if on_dev else out.cpu().numpy()
 
     def min_distance_from(self, p) -> float:
@@ -107,16 +125,11 @@ class Shape:
     def batch_contains(self, points):
         """Shape::contains (src/shape/mod.rs:78-80) for many points (bool)."""
         torch = _torch()
-        lib = load()
-        on_dev = isinstance(points, torch.Tensor) and points.is_cuda
-        pts = points if on_dev else torch.as_tensor(np.ascontiguousarray(points, np.float32))
-        pts = pts.reshape(-1, 3).to(device="cuda" if not on_dev else pts.device,
-                                    dtype=torch.float32).contiguous()
+        on_dev, pts = _device_points(torch, points)
         out = torch.empty(pts.shape[0], dtype=torch.uint8, device=pts.device)
-        with torch.cuda.device(pts.device):
-            check(lib.cg_contains(C.byref(self._cshape()), C.c_void_p(pts.data_ptr()),
-                                  pts.shape[0], C.c_void_p(out.data_ptr()),
-                                  _stream_ptr(pts.device)))
+        with _on_device(torch, pts.device):
+            check(load().cg_contains(C.byref(self._cshape()), pts.data_ptr(), pts.shape[0],
+                                     out.data_ptr(), _stream_ptr(pts.device)))
         res = out.bool()
         return res if on_dev else res.cpu().numpy()
 

@@ -33,6 +33,17 @@ def _shape(power: float, rot, max_iters: int, bailout: float) -> _ffi.CgShape:
     return s
 
 
+def split_params(params, power_device, rot_device):
+    """(d/dpower, d/drotation) of a 4-vector of parameter gradients on the
+    parameters' devices, in one transfer where they share one."""
+    def move(t, device):
+        return t if device is None else t.to(device)
+
+    if power_device == rot_device:
+        params = move(params, power_device)
+    return move(params[0], power_device), move(params[1:4], rot_device)
+
+
 def _make_function():
     torch = _torch()
 
@@ -40,8 +51,7 @@ def _make_function():
         @staticmethod
         def forward(ctx, points, power, rot, max_iters, bailout):
             pts = points.detach().contiguous().float()
-            shape = _shape(float(power), [float(r) for r in rot.detach().cpu()], max_iters,
-                           bailout)
+            shape = _shape(float(power), rot.detach().reshape(-1).tolist(), max_iters, bailout)
             out = torch.empty(pts.shape[0], dtype=torch.float32, device=pts.device)
             stream = torch.cuda.current_stream(pts.device)
             check(load().cg_min_distance_from(C.byref(shape), C.c_void_p(pts.data_ptr()),
@@ -66,10 +76,9 @@ def _make_function():
                                         C.c_void_p(gp.data_ptr()) if gp is not None else None,
                                         C.c_void_p(params.data_ptr()),
                                         C.c_void_p(stream.cuda_stream)))
-            pdev, rdev = ctx.param_devices
-            gpow = params[0].to(pdev) if ctx.needs_input_grad[1] else None
-            grot = params[1:4].to(rdev) if ctx.needs_input_grad[2] else None
-            return gp, gpow, grot, None, None
+            gpow, grot = split_params(params, *ctx.param_devices)
+            return (gp, gpow if ctx.needs_input_grad[1] else None,
+                    grot if ctx.needs_input_grad[2] else None, None, None)
 
     return MandelbulbDE
 

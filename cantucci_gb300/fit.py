@@ -30,6 +30,7 @@ import math
 
 from . import _ffi
 from ._ffi import check, load
+from .autograd import split_params
 
 
 def _torch():
@@ -87,7 +88,7 @@ def _make_render_fn():
         @staticmethod
         def forward(ctx, power, rot, cam, max_steps, eps_scale, max_iters, bailout, fast, cap):
             p = float(power)
-            r = [float(v) for v in rot.detach().cpu()]
+            r = rot.detach().reshape(-1).tolist()
             depth = render(p, r, cam, max_steps, eps_scale, max_iters, bailout, fast=fast)
             ctx.save_for_backward(depth)
             ctx.shape = _shape(p, r, max_iters, bailout)
@@ -106,8 +107,7 @@ def _make_render_fn():
                 C.byref(ctx.shape), C.byref(ctx.cam), C.c_void_p(depth.data_ptr()),
                 C.c_void_p(g.data_ptr()), ctx.cap, C.c_void_p(params.data_ptr()),
                 C.c_void_p(torch.cuda.current_stream().cuda_stream)))
-            pdev, rdev = ctx.param_devices
-            return (params[0].to(pdev), params[1:4].to(rdev), None, None, None, None, None,
+            return (*split_params(params, *ctx.param_devices), None, None, None, None, None,
                     None, None)
 
     return DepthRender
@@ -180,8 +180,7 @@ def _make_surface_fn():
         def forward(ctx, power, rot, points, max_iters, bailout, cap):
             pts = points.contiguous().float()
             out = torch.empty(5, dtype=torch.float32, device=pts.device)
-            shape = _shape(float(power), [float(v) for v in rot.detach().cpu()], max_iters,
-                           bailout)
+            shape = _shape(float(power), rot.detach().reshape(-1).tolist(), max_iters, bailout)
             check(load().cg_surface_l1(
                 C.byref(shape), C.c_void_p(pts.data_ptr()), pts.shape[0], max(float(cap), 0.0),
                 C.c_void_p(out.data_ptr()),
@@ -194,9 +193,7 @@ def _make_surface_fn():
         @staticmethod
         def backward(ctx, gout):
             (grad,) = ctx.saved_tensors
-            pdev, rdev = ctx.devs
-            return ((gout * grad[0]).to(pdev), (gout * grad[1:4]).to(rdev), None, None, None,
-                    None)
+            return (*split_params(gout * grad, *ctx.devs), None, None, None, None)
 
     return SurfaceL1
 
