@@ -264,7 +264,6 @@ cg_status enqueue_mesh(cg_mesher* m, const ShapeDev& s, const SpanSetup& su, con
                                 cudaMemcpyHostToDevice, st));
     cudaStream_t ts = m->timing_stream;
     CG_CUDA(record_event(m->ev[0], st, ts, m->timing_fork));
-    CG_CUDA(cudaMemsetAsync(w.sgn, 0, ((size_t)d.n * d.n * d.W + 1) * sizeof(uint32_t), st));
     CG_TRY(launch_de_grid(s, make_grid(su, d.res), w.dists, m->numerics, st, w.sgn, d.W,
                           dp ? &dp->g : nullptr));
     CG_CUDA(record_event(m->ev[1], st, ts, m->timing_fork));
@@ -413,7 +412,6 @@ cg_status run_mesh_to_host(cg_mesher* m, const cg_span* span, const cg_shape* sh
     mesh_workspace_layout(res, m->work, &w);
     cudaStream_t st = m->stream;
     CG_CUDA(cudaEventRecord(m->ev[0], st));
-    CG_CUDA(cudaMemsetAsync(w.sgn, 0, ((size_t)d.n * d.n * d.W + 1) * sizeof(uint32_t), st));
     CG_TRY(launch_de_grid(s, make_grid(su, res), w.dists, m->numerics, st, w.sgn, d.W));
     CG_CUDA(cudaEventRecord(m->ev[1], st));
     CG_TRY(launch_mesh_to_host(s, su, d, w, hverts_dev, vcap, m->didx, hidx, idev, st,

@@ -106,32 +106,41 @@ struct GridCoord {
 };
 
 // Grids of res 32 and 64, one brick or face item to a warp: the lanes of
-// k_de_grid_units without its walk, in fewer registers.
+// k_de_grid_units without its walk, in fewer registers.  A block is a core unit
+// (its eight bricks' ballots meet in shared memory as the rows' sign words) or
+// eight face items, so every sign word is stored whole.
 template <int M>
-__global__ void __launch_bounds__(128, 10) k_de_grid_small(ShapeDev s, GridDev g,
-                                                           float* __restrict__ out,
-                                                           uint32_t* __restrict__ sgn, uint32_t W,
-                                                           uint32_t shift,
-                                                           const GridDev* __restrict__ gp) {
+__global__ void __launch_bounds__(256, 5) k_de_grid_small(ShapeDev s, GridDev g,
+                                                          float* __restrict__ out,
+                                                          uint32_t* __restrict__ sgn, uint32_t W,
+                                                          uint32_t shift,
+                                                          const GridDev* __restrict__ gp) {
+    __shared__ uint32_t ballots[8];
     if (gp) g = *gp;
     const GridCoord coord{g};
-    const uint32_t n = g.n, lane = threadIdx.x & 31;
-    const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, bricks = core_bricks(shift);
-    if (c >= bricks) {
-        if (c - bricks < face_items(shift)) face_item<M>(s, coord, shift, W, c - bricks, out, sgn);
+    const uint32_t n = g.n, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t core = core_units(shift);
+    if (blockIdx.x >= core) {
+        const uint32_t f = 8 * (blockIdx.x - core) + warp;
+        if (f < face_items(shift)) face_item<M>(s, coord, shift, W, f, out, sgn);
         return;
     }
-    const uint32_t mask = (1u << (shift - 2)) - 1u, t = c >> (shift - 2);
-    const uint32_t x = 2 * (t >> (shift - 2)) + (lane >> 4), y = 4 * (t & mask) + ((lane >> 2) & 3),
-                   z = 4 * (c & mask) + (lane & 3);
+    const uint32_t c = blockIdx.x, gz = c & ((1u << (shift - 5)) - 1u), t = c >> (shift - 5);
+    const uint32_t x0 = 2 * (t >> (shift - 2)), y0 = 4 * (t & ((1u << (shift - 2)) - 1u));
+    const uint32_t x = x0 + (lane >> 4), y = y0 + ((lane >> 2) & 3);
+    const uint32_t z = 32 * gz + 4 * warp + (lane & 3);
     const float d = eval<M>(s, coord(0, x), coord(1, y), coord(2, z));
     CG_AT(out, ((size_t)x * n + y) * n + z, (uint64_t)n * n * n) = d;
-    if (sgn) {
-        const uint32_t b = __ballot_sync(0xFFFFFFFFu, (__float_as_uint(d) >> 31) == 0u);
-        const uint32_t bits = (b >> (lane & ~3u)) & 0xFu;
-        if ((lane & 3) == 0 && bits)
-            atomicOr(&CG_AT(sgn, (x * n + y) * W + (z >> 5), (uint64_t)n * n * W),
-                     bits << (z & 31));
+    if (!sgn) return;
+    const uint32_t b = __ballot_sync(0xFFFFFFFFu, (__float_as_uint(d) >> 31) == 0u);
+    if (lane == 0) ballots[warp] = b;
+    __syncthreads();
+    if (threadIdx.x < 8) {  // row k of the unit's 2 x 4: bits 4 k of each ballot
+        const uint32_t k = threadIdx.x;
+        uint32_t word = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < 8; ++w) word |= ((ballots[w] >> (4 * k)) & 0xFu) << (4 * w);
+        CG_AT(sgn, ((x0 + (k >> 2)) * n + y0 + (k & 3)) * W + gz, (uint64_t)n * n * W) = word;
     }
 }
 
@@ -447,21 +456,29 @@ int set_de_grid_kernel(int v) {
 }
 
 template <int M>
-static void launch_grid_mode(const ShapeDev& s, const GridDev& g, float* out, uint32_t* sgn,
-                             uint32_t W, cudaStream_t st, const GridDev* gp) {
+static cg_status launch_grid_mode(const ShapeDev& s, const GridDev& g, float* out, uint32_t* sgn,
+                                  uint32_t W, cudaStream_t st, const GridDev* gp) {
     const unsigned B = 256;
     int k = g_de_grid_kernel;
+    const bool automatic = k == DE_GRID_AUTO;
+    const size_t words = (size_t)g.n * g.n * W;
+    // The kernels that set single bits of a sign word want the words zeroed.
+    auto clear = [&](uint32_t* p, size_t count) -> cg_status {
+        if (sgn) CG_CUDA(cudaMemsetAsync(p, 0, count * sizeof(uint32_t), st));
+        return CG_OK;
+    };
     // Up to 65^3 corners (res 64, cantucci's leaves) one brick to a warp: the
     // brick walk's 63 registers (4 blocks of 256 threads per SM) would fit the
-    // grid in more waves than k_de_grid_small's 44, and one corner per thread
-    // in row order keeps 24 lanes busy against 27 (15.8 against 14.7 us).
-    if (k == DE_GRID_AUTO) k = g.n > 65 ? DE_GRID_BRICK : DE_GRID_LINEAR;
+    // grid in more waves than k_de_grid_small's, and one corner per thread in
+    // row order keeps 24 lanes busy against 27 (15.8 against 14.7 us).
+    if (automatic) k = g.n > 65 ? DE_GRID_BRICK : DE_GRID_LINEAR;
     uint32_t shift = 0;
     while ((2u << shift) < g.n) ++shift;
-    if (g_de_grid_kernel == DE_GRID_AUTO && k == DE_GRID_LINEAR && g.n > kUnitMinRes) {
-        const uint32_t warps = core_bricks(shift) + face_items(shift);
-        k_de_grid_small<M><<<(warps + 3) / 4, 128, 0, st>>>(s, g, out, sgn, W, shift, gp);
+    if (automatic && k == DE_GRID_LINEAR && g.n > kUnitMinRes) {
+        const uint32_t blocks = core_units(shift) + (face_items(shift) + 7) / 8;
+        k_de_grid_small<M><<<blocks, B, 0, st>>>(s, g, out, sgn, W, shift, gp);
     } else if (k == DE_GRID_PACKED && (M == MODE_P8 || M == MODE_P8_IT15)) {
+        CG_TRY(clear(sgn, words));
         const uint64_t b4 = (g.n + 3) >> 2;
         k_de_grid_p8x2<<<grid_for(b4 * b4 * b4 * 32, B, 8), B, 0, st>>>(s, g, out, sgn, W, gp);
     } else if (k != DE_GRID_LINEAR) {
@@ -472,33 +489,37 @@ static void launch_grid_mode(const ShapeDev& s, const GridDev& g, float* out, ui
         const uint64_t units8 = rows * ((bz + 7) / 8);
         if (units8 >= 4ull * sm_count() * 8 * (B / 32)) {
             const uint64_t units = core_units(shift) + (face_items(shift) + 7) / 8;
-            uint32_t* queue = sgn ? sgn + (size_t)g.n * g.n * W : nullptr;
-            k_de_grid_units<M><<<grid_for(units * 32, B, 8), B, 0, st>>>(
-                s, g, out, sgn, W, shift, queue, gp);
+            uint32_t* queue = sgn ? sgn + words : nullptr;
+            CG_TRY(clear(queue, 1));
+            k_de_grid_units<M><<<grid_for(units * 32, B, 8), B, 0, st>>>(s, g, out, sgn, W, shift,
+                                                                         queue, gp);
         } else {
+            CG_TRY(clear(sgn, words));
             k_de_grid_brick<M><<<grid_for(rows * bz * 32, B, 8), B, 0, st>>>(s, g, out, sgn, W, gp);
         }
     } else {
+        CG_TRY(clear(sgn, words));
         const uint64_t total = (uint64_t)g.n * g.n * g.n;
         k_de_grid<M><<<grid_for(total, B, 8), B, 0, st>>>(s, g, out, sgn, W, gp);
     }
+    return CG_OK;
 }
 
 cg_status launch_de_grid(const ShapeDev& s, const GridDev& g, float* out, uint32_t numerics,
                          cudaStream_t st, uint32_t* sgn, uint32_t W, const GridDev* gp) {
     switch (mode_of(s, numerics)) {
     case MODE_P8:
-        if (p8_unrolled(s)) launch_grid_mode<MODE_P8_IT15>(s, g, out, sgn, W, st, gp);
-        else launch_grid_mode<MODE_P8>(s, g, out, sgn, W, st, gp);
+        if (p8_unrolled(s)) CG_TRY(launch_grid_mode<MODE_P8_IT15>(s, g, out, sgn, W, st, gp));
+        else CG_TRY(launch_grid_mode<MODE_P8>(s, g, out, sgn, W, st, gp));
         break;
-    case MODE_INT: launch_grid_mode<MODE_INT>(s, g, out, sgn, W, st, gp); break;
-    case MODE_POLAR: launch_grid_mode<MODE_POLAR>(s, g, out, sgn, W, st, gp); break;
-    case MODE_SPHERE: launch_grid_mode<MODE_SPHERE>(s, g, out, sgn, W, st, gp); break;
-    case MODE_INT_POLY: launch_grid_mode<MODE_INT_POLY>(s, g, out, sgn, W, st, gp); break;
-    case MODE_POLAR_FAST: launch_grid_mode<MODE_POLAR_FAST>(s, g, out, sgn, W, st, gp); break;
+    case MODE_INT: CG_TRY(launch_grid_mode<MODE_INT>(s, g, out, sgn, W, st, gp)); break;
+    case MODE_POLAR: CG_TRY(launch_grid_mode<MODE_POLAR>(s, g, out, sgn, W, st, gp)); break;
+    case MODE_SPHERE: CG_TRY(launch_grid_mode<MODE_SPHERE>(s, g, out, sgn, W, st, gp)); break;
+    case MODE_INT_POLY: CG_TRY(launch_grid_mode<MODE_INT_POLY>(s, g, out, sgn, W, st, gp)); break;
+    case MODE_POLAR_FAST: CG_TRY(launch_grid_mode<MODE_POLAR_FAST>(s, g, out, sgn, W, st, gp)); break;
     default:
-        if (p8_unrolled(s)) launch_grid_mode<MODE_P8_FAST_IT15>(s, g, out, sgn, W, st, gp);
-        else launch_grid_mode<MODE_P8_FAST>(s, g, out, sgn, W, st, gp);
+        if (p8_unrolled(s)) CG_TRY(launch_grid_mode<MODE_P8_FAST_IT15>(s, g, out, sgn, W, st, gp));
+        else CG_TRY(launch_grid_mode<MODE_P8_FAST>(s, g, out, sgn, W, st, gp));
         break;
     }
     CG_CHECK_LAUNCH("k_de_grid");

@@ -46,9 +46,9 @@ int set_de_grid_kernel(int v);
 int de_grid_kernel_option();
 uint32_t place_blocks_per_sm();
 
-// Step 1 on a span grid.  With `sgn` (zeroed, (res+1)^2 rows x W words, and one
-// word more for a work queue) the kernel also packs is_sign_positive of every
-// corner into sign words.
+// Step 1 on a span grid.  With `sgn` ((res+1)^2 rows x W words, and one word more
+// for a work queue) the kernel also packs is_sign_positive of every corner into
+// sign words; what it needs zeroed there is zeroed first.
 // With `gp` the kernels take the grid from device memory instead of `g`
 // (which still fixes the launch shape): a captured graph then serves every
 // span of the same resolution.
