@@ -44,17 +44,23 @@ __global__ void __launch_bounds__(128) k_de_grad(ShapeDev s, Dm3 dm, const float
 }
 
 // The same over the long tape (max_iters <= ADJ_LONG_MAX).
-__global__ void __launch_bounds__(ADJ_LONG_BLOCK) k_de_grad_long(ShapeDev s, Dm3 dm,
-                                                                 const float* __restrict__ pts,
-                                                                 uint64_t n,
-                                                                 float* __restrict__ out) {
-    extern __shared__ __align__(16) float long_smem[];
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+__global__ void __launch_bounds__(ADJ_BLOCK, LONG_BLOCKS) k_de_grad_long(ShapeDev s, Dm3 dm,
+                                                            const float* __restrict__ pts,
+                                                            uint64_t n, float* __restrict__ out) {
+    extern __shared__ __align__(16) float4 adj_smem[];
+    __shared__ uint32_t slot;
+    const LongTape tape = long_tape_open(reinterpret_cast<float*>(adj_smem), &slot,
+                                         long_tape_columns(s.max_iters));
+    const WarpWalk w = warp_walk();
+    for (uint64_t base = w.first; base < n; base += w.stride) {
+        const uint64_t i = base + (threadIdx.x & 31);
+        const bool in = i < n;
+        const float* p = pts + 3 * (in ? i : base);
         float o[8];
-        polar_de_grad_long(s, dm.m, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], long_smem, o);
-        store8(out, i, o);
+        polar_de_grad_long(s, dm.m, in, p[0], p[1], p[2], tape, o);
+        if (in) store8(out, i, o);
     }
+    long_tape_close(&slot, long_tape_columns(s.max_iters));
 }
 
 template <int T, bool FAST>
@@ -98,8 +104,8 @@ __global__ void __launch_bounds__(128) k_de_spatial_grad(ShapeDev s, const float
 }
 
 // Vector-Jacobian product of a batch: g[i] * dDE/dp into grad_points (n x 3)
-// and, per warp, the sum over its points of g[i] * dDE/d(power, euler), in
-// double, into partial[4 w .. 4 w + 3] (added up by k_sum_partials4 in a fixed
+// and, per block, the sum over its points of g[i] * dDE/d(power, euler), in
+// double, into params[4 b .. 4 b + 3] (added up by k_sum_partials4 in a fixed
 // order, so the result does not depend on scheduling; the terms of chaotic
 // points cancel over ten decades).
 template <bool LONG>
@@ -107,15 +113,23 @@ __global__ void __launch_bounds__(128) k_de_vjp(ShapeDev s, Dm3 dm, const float*
                                                 const float* __restrict__ g, uint64_t n,
                                                 float* __restrict__ gp, double* __restrict__ params) {
     extern __shared__ __align__(16) float4 adj_smem[];
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    __shared__ uint32_t slot;
+    const uint32_t columns = long_tape_columns(s.max_iters);
+    LongTape tape;
+    if constexpr (LONG) tape = long_tape_open(reinterpret_cast<float*>(adj_smem), &slot, columns);
+    const WarpWalk walk = warp_walk();
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    for (uint64_t base = walk.first; base < n; base += walk.stride) {
+        const uint64_t i = base + (threadIdx.x & 31);
+        const bool in = i < n;
+        const float* p = pts + 3 * (in ? i : base);
         float o[8];
-        const float x = pts[3 * i], y = pts[3 * i + 1], z = pts[3 * i + 2];
         if constexpr (LONG)
-            polar_de_grad_long(s, dm.m, x, y, z, reinterpret_cast<float*>(adj_smem), o);
-        else
-            polar_de_grad<ADJ_CK>(s, dm.m, x, y, z, adj_tape(adj_smem, s.max_iters, ADJ_CK), o);
+            polar_de_grad_long(s, dm.m, in, p[0], p[1], p[2], tape, o);
+        else if (in)
+            polar_de_grad<ADJ_CK>(s, dm.m, p[0], p[1], p[2],
+                                  adj_tape(adj_smem, s.max_iters, ADJ_CK), o);
+        if (!in) continue;
         const float gi = g[i];
         if (gp) {
             gp[3 * i] = gi * o[1];
@@ -130,26 +144,19 @@ __global__ void __launch_bounds__(128) k_de_vjp(ShapeDev s, Dm3 dm, const float*
             }
         }
     }
-    if (params) {
-        const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            double v = acc[k];
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, o);
-            if ((threadIdx.x & 31) == 0) params[4 * w + k] = v;
-        }
-    }
+    if constexpr (LONG) long_tape_close(&slot, columns);
+    if (params) block_sums(acc, params);
 }
 
-// params[k] = the sum over warps w < nwarps of partial[4 w + k], in a fixed
+// params[k] = the sum over blocks b < blocks of partial[4 b + k], in a fixed
 // order: strided sequential sums, eight warps to a column, then a fixed tree.
 __global__ void __launch_bounds__(1024) k_sum_partials4(const double* __restrict__ partial,
-                                                        uint32_t nwarps,
+                                                        uint32_t blocks,
                                                         float* __restrict__ params) {
     __shared__ double sh[32];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = warp & 3;
     double v = 0.0;
-    for (uint32_t w = (warp >> 2) * 32 + lane; w < nwarps; w += 256) v += partial[4 * w + k];
+    for (uint32_t b = (warp >> 2) * 32 + lane; b < blocks; b += 256) v += partial[4 * b + k];
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, o);
     if (lane == 0) sh[warp] = v;
     __syncthreads();
@@ -162,7 +169,7 @@ __global__ void __launch_bounds__(1024) k_sum_partials4(const double* __restrict
 
 // Mean |DE| over the points whose DE and derivatives are all finite, and its
 // gradient with respect to (power, euler) without the points of which some
-// |dDE/dtheta_k| exceeds cap (0: none): per warp the sums (points, |DE|, four
+// |dDE/dtheta_k| exceeds cap (0: none): per block the sums (points, |DE|, four
 // derivatives) in double, added up in a fixed order by k_surface_l1_sum.  One
 // pass over the points in place of the gradients of all of them, a dozen
 // reductions and selections on those and the synchronisations that selecting
@@ -173,16 +180,24 @@ __global__ void __launch_bounds__(128) k_surface_l1(ShapeDev s, Dm3 dm,
                                                     const float* __restrict__ pts, uint64_t n,
                                                     float cap, double* __restrict__ partial) {
     extern __shared__ __align__(16) float4 adj_smem[];
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    __shared__ uint32_t slot;
+    const uint32_t columns = long_tape_columns(s.max_iters);
+    LongTape tape;
+    if constexpr (MODE == 0)
+        tape = long_tape_open(reinterpret_cast<float*>(adj_smem), &slot, columns);
+    const WarpWalk walk = warp_walk();
     double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    for (uint64_t base = walk.first; base < n; base += walk.stride) {
+        const uint64_t i = base + (threadIdx.x & 31);
+        const bool in = i < n;
+        const float* p = pts + 3 * (in ? i : base);
         float o[8];
-        const float x = pts[3 * i], y = pts[3 * i + 1], z = pts[3 * i + 2];
         if constexpr (MODE == 0)
-            polar_de_grad_long(s, dm.m, x, y, z, reinterpret_cast<float*>(adj_smem), o);
-        else
-            polar_de_grad<ADJ_CK, MODE == 2>(s, dm.m, x, y, z,
+            polar_de_grad_long(s, dm.m, in, p[0], p[1], p[2], tape, o);
+        else if (in)
+            polar_de_grad<ADJ_CK, MODE == 2>(s, dm.m, p[0], p[1], p[2],
                                              adj_tape(adj_smem, s.max_iters, ADJ_CK), o);
+        if (!in) continue;
         bool ok = true, keep = true;
 #pragma unroll
         for (int k = 0; k < 8; ++k) ok = ok && isfinite(o[k]);
@@ -195,27 +210,23 @@ __global__ void __launch_bounds__(128) k_surface_l1(ShapeDev s, Dm3 dm,
 #pragma unroll
             for (int k = 0; k < 4; ++k) acc[2 + k] += o[0] > 0.0f ? o[4 + k] : -o[4 + k];
     }
-    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        double v = acc[k];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, o);
-        if ((threadIdx.x & 31) == 0) partial[6 * w + k] = v;
-    }
+    if constexpr (MODE == 0) long_tape_close(&slot, columns);
+    block_sums(acc, partial);
 }
 
-// out = (mean |DE|, its four derivatives): warp k of one block sums column k
-// over the nwarps partial sums, in a fixed order.
-__global__ void __launch_bounds__(192) k_surface_l1_sum(const double* __restrict__ partial,
-                                                        uint32_t nwarps, float* __restrict__ out) {
-    __shared__ double sums[6];
-    const uint32_t lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+// out = (mean |DE|, its four derivatives): four warps of one block to a column
+// of the blocks' partial sums, added up in a fixed order.
+__global__ void __launch_bounds__(768) k_surface_l1_sum(const double* __restrict__ partial,
+                                                        uint32_t blocks, float* __restrict__ out) {
+    __shared__ double sh[24];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = warp % 6;
     double v = 0.0;
-    for (uint32_t w = lane; w < nwarps; w += 32) v += partial[6 * w + k];
+    for (uint32_t b = (warp / 6) * 32 + lane; b < blocks; b += 128) v += partial[6 * b + k];
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, o);
-    if (lane == 0) sums[k] = v;
+    if (lane == 0) sh[warp] = v;
     __syncthreads();
-    if (threadIdx.x < 5) out[threadIdx.x] = (float)(sums[1 + threadIdx.x] / fmax(sums[0], 1.0));
+    const auto column = [&](int c) { return ((sh[c] + sh[6 + c]) + sh[12 + c]) + sh[18 + c]; };
+    if (threadIdx.x < 5) out[threadIdx.x] = (float)(column(1 + threadIdx.x) / fmax(column(0), 1.0));
 }
 
 // The calling thread's partials buffer on the current device, grown as
@@ -281,9 +292,9 @@ cg_status release_partials(float* partial, cudaStream_t st) {
     return CG_OK;
 }
 
-cg_status launch_sum_partials4(const float* partial, uint32_t nwarps, float* params,
+cg_status launch_sum_partials4(const float* partial, uint32_t blocks, float* params,
                                cudaStream_t st) {
-    k_sum_partials4<<<1, 1024, 0, st>>>(reinterpret_cast<const double*>(partial), nwarps, params);
+    k_sum_partials4<<<1, 1024, 0, st>>>(reinterpret_cast<const double*>(partial), blocks, params);
     CG_CHECK_LAUNCH("k_sum_partials4");
     return CG_OK;
 }
@@ -372,9 +383,9 @@ static cg_status launch_de_grad(const ShapeDev& sd, const Dm3& dm, uint32_t max_
                                 const float* points, uint64_t n, float* out, cudaStream_t st) {
     unsigned G = 0;
     if (CK == ADJ_CK && !FR && max_iters <= ADJ_LONG_MAX) {
-        const size_t smem = long_tape_bytes(max_iters, ADJ_LONG_BLOCK);
-        CG_TRY(adj_launch_shape(k_de_grad_long, ADJ_LONG_BLOCK, smem, n, &G));
-        k_de_grad_long<<<G, ADJ_LONG_BLOCK, smem, st>>>(sd, dm, points, n, out);
+        size_t smem = 0;
+        CG_TRY(long_launch_shape(k_de_grad_long, max_iters, n, &smem, &G));
+        k_de_grad_long<<<G, ADJ_BLOCK, smem, st>>>(sd, dm, points, n, out);
         CG_CHECK_LAUNCH("k_de_grad_long");
         return CG_OK;
     }
@@ -480,19 +491,17 @@ cg_status cg_de_backward(const cg_shape* shape, const float* points, const float
         return CG_OK;
     }
     const bool lng = shape->max_iters <= ADJ_LONG_MAX;
-    const unsigned B = lng ? ADJ_LONG_BLOCK : ADJ_BLOCK;
-    const size_t smem = lng ? long_tape_bytes(shape->max_iters, B)
-                            : adj_tape_bytes(shape->max_iters, ADJ_CK, B);
+    size_t smem = adj_tape_bytes(shape->max_iters, ADJ_CK, ADJ_BLOCK);
     auto kernel = lng ? k_de_vjp<true> : k_de_vjp<false>;
     unsigned G = 0;
-    CG_TRY(adj_launch_shape(kernel, B, smem, n, &G));
-    const uint32_t nwarps = G * (B / 32);
+    CG_TRY(lng ? long_launch_shape(kernel, shape->max_iters, n, &smem, &G)
+               : adj_launch_shape(kernel, ADJ_BLOCK, smem, n, &G));
     float* partial = nullptr;
-    if (grad_params) CG_TRY(acquire_partials((size_t)nwarps * 8, st, &partial));
-    kernel<<<G, B, smem, st>>>(make_shape_dev(*shape), rotation_derivatives(*shape), points,
+    if (grad_params) CG_TRY(acquire_partials((size_t)G * 8, st, &partial));
+    kernel<<<G, ADJ_BLOCK, smem, st>>>(make_shape_dev(*shape), rotation_derivatives(*shape), points,
                                grad_out, n, grad_points, reinterpret_cast<double*>(partial));
     cg_status rs = cuda_status(cudaGetLastError(), "k_de_vjp", __FILE__, __LINE__);
-    if (rs == CG_OK && partial) rs = launch_sum_partials4(partial, nwarps, grad_params, st);
+    if (rs == CG_OK && partial) rs = launch_sum_partials4(partial, G, grad_params, st);
     if (partial) {
         const cg_status rr = release_partials(partial, st);
         if (rs == CG_OK) rs = rr;
@@ -508,21 +517,19 @@ cg_status cg_surface_l1(const cg_shape* shape, const float* points, uint64_t n, 
         return CG_EINVAL;
     }
     const bool lng = g_adjoint_fastrec == 0 && shape->max_iters <= ADJ_LONG_MAX;
-    const unsigned B = lng ? ADJ_LONG_BLOCK : ADJ_BLOCK;
-    const size_t smem = lng ? long_tape_bytes(shape->max_iters, B)
-                            : adj_tape_bytes(shape->max_iters, ADJ_CK, B);
+    size_t smem = adj_tape_bytes(shape->max_iters, ADJ_CK, ADJ_BLOCK);
     auto kernel = lng ? k_surface_l1<0> : (g_adjoint_fastrec ? k_surface_l1<2> : k_surface_l1<1>);
     cudaStream_t st = (cudaStream_t)stream;
     unsigned G = 0;
-    CG_TRY(adj_launch_shape(kernel, B, smem, n, &G));
-    const uint32_t nwarps = G * (B / 32);
+    CG_TRY(lng ? long_launch_shape(kernel, shape->max_iters, n, &smem, &G)
+               : adj_launch_shape(kernel, ADJ_BLOCK, smem, n, &G));
     float* partial = nullptr;
-    CG_TRY(acquire_partials((size_t)nwarps * 12, st, &partial));
-    kernel<<<G, B, smem, st>>>(make_shape_dev(*shape), rotation_derivatives(*shape), points, n, cap,
-                               reinterpret_cast<double*>(partial));
+    CG_TRY(acquire_partials((size_t)G * 12, st, &partial));
+    kernel<<<G, ADJ_BLOCK, smem, st>>>(make_shape_dev(*shape), rotation_derivatives(*shape), points, n,
+                                       cap, reinterpret_cast<double*>(partial));
     cg_status rs = cuda_status(cudaGetLastError(), "k_surface_l1", __FILE__, __LINE__);
     if (rs == CG_OK) {
-        k_surface_l1_sum<<<1, 192, 0, st>>>(reinterpret_cast<double*>(partial), nwarps, out);
+        k_surface_l1_sum<<<1, 768, 0, st>>>(reinterpret_cast<double*>(partial), G, out);
         rs = cuda_status(cudaGetLastError(), "k_surface_l1_sum", __FILE__, __LINE__);
     }
     const cg_status rr = release_partials(partial, st);

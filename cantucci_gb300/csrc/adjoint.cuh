@@ -7,12 +7,13 @@
 // For the polar loop one thread returns, per point,
 //   DE, dDE/dp (3), dDE/dpower, dDE/d(euler angles) (3).
 // It is the adjoint of the forward loop, not a finite difference: the
-// forward pass keeps a checkpoint of (z, dr) every CK steps and the step
-// records of its last segment in a per-thread tape in shared memory (never
-// in HBM or local memory); the backward pass walks the segments from last to
-// first, recomputes each earlier segment's iterates from its checkpoint and
-// back-propagates through them.  Work is one forward pass, the recompute of
-// all steps but the last segment's, and one backward pass.
+// forward pass keeps every step's record in a per-thread tape in shared and
+// tensor memory (loops of up to ADJ_LONG_MAX steps), or a checkpoint of (z, dr)
+// every CK steps and the records of its last segment in shared memory; never
+// in HBM or local memory.  With checkpoints the backward pass walks the
+// segments from last to first, recomputes each earlier segment's iterates and
+// back-propagates through them: one forward pass, the recompute of all steps
+// but the last segment's, and one backward pass.
 //
 // Per step k (z_k -> z_{k+1} = r^P u(P theta, P phi) + q, dr_{k+1} =
 // r^(P-1) P dr_k + 1, r = |z_k|, theta = acos(z_z / r), phi = atan2(y, x)):
@@ -167,19 +168,100 @@ __device__ __forceinline__ StepDeriv tape_get(const AdjTape& t, uint32_t slot) {
 }
 
 // The long tape: of every step what the backward sweep cannot form again from
-// its neighbours -- dr, r^(P-1), the two angles, r^P and the sines and cosines
-// (z_k follows from step k - 1's record and q by the step's own operations, r
-// from z_k).  The last step the loop allows needs the first two only.  No
-// checkpoints and no recomputed segments, 512 bytes per thread at 15 steps.
-constexpr int LONG_FIELDS = 9;
+// its neighbours -- dr, r^(P-1), the two angles and r^P in shared memory, the
+// sines and cosines in tensor memory (z_k follows from step k - 1's record and
+// q by the step's own operations, r from z_k).  The last step the loop allows
+// needs the first two only.  No checkpoints and no recomputed segments.
+//
+// Tensor memory is 256 KB per SM that nothing else here uses: a thread's row of
+// it (its lane in its warp's quarter) holds four columns per step.  With all
+// nine values in shared memory 12 warps fit an SM at 15 steps and the kernels
+// issued 65 % of the time; with five, 24 do, 80 %.  Gradients of 2 M points near
+// the surface at 15 steps 555 -> 430 us, at 10 steps 328 -> 285; batch products
+// with their sums, 1 M points, 285 -> 235; the depth map's backward pass,
+// 512 x 512, 77 -> 64; up to 20 K points the same (latency).
+constexpr int LONG_FIELDS = 5;
 constexpr uint32_t ADJ_LONG_MAX = 20;  // the longest loop that takes it
 
-__host__ __device__ constexpr size_t long_tape_bytes(uint32_t max_iters, uint32_t nth) {
-    return ((size_t)LONG_FIELDS * (max_iters - 1) + 2u) * 4u * nth;
+// Columns for the sines and cosines of max_iters - 1 steps: a power of two.
+__host__ __device__ constexpr uint32_t long_tape_columns(uint32_t max_iters) {
+    return max_iters <= 9 ? 32u : (max_iters <= 17 ? 64u : 128u);
 }
 
-constexpr unsigned ADJ_BLOCK = 128;      // threads per block, checkpointed tape
-constexpr unsigned ADJ_LONG_BLOCK = 64;  // long tape
+constexpr unsigned ADJ_BLOCK = 128;  // threads per block: a warp per quarter of tensor memory
+
+constexpr unsigned LONG_BLOCKS = 7;  // most blocks per SM: 72 registers a thread
+// Blocks launched for each that fits: the SMs even out what one of them is late
+// (2 M points: 467 us at 1, 444 at 2, 430 at 4 and 425 at 16, but 16 times the
+// partial sums cost the sums 17 us more).
+constexpr unsigned LONG_WAVES = 4;
+
+// Dynamic shared memory of a block; never so little that more than LONG_BLOCKS
+// blocks (at more than 64 columns 4) share an SM's 228 KB, of which every block
+// takes 1 KB more, since a block that finds its SM's 512 columns taken waits
+// for another to end.
+__host__ __device__ constexpr size_t long_tape_bytes(uint32_t max_iters) {
+    const size_t b = ((size_t)LONG_FIELDS * (max_iters - 1) + 2u) * 4u * ADJ_BLOCK;
+    const size_t least = long_tape_columns(max_iters) > 64u ? 46u * 1024u : 30u * 1024u;
+    return b < least ? least : b;
+}
+
+struct LongTape {
+    float* smem;    // this thread's first word; fields ADJ_BLOCK apart
+    uint32_t tmem;  // this warp's tensor memory address
+};
+
+// Allocates the block's columns (all its threads call, once).
+__device__ __forceinline__ LongTape long_tape_open(float* smem, uint32_t* slot, uint32_t columns) {
+    const uint32_t warp = threadIdx.x >> 5;
+    if (warp == 0) {
+        const uint32_t at = (uint32_t)__cvta_generic_to_shared(slot);
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(at),
+                     "r"(columns)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    return {smem + threadIdx.x, *slot + (warp << 21)};  // lanes 32 w of the block's columns
+}
+
+__device__ __forceinline__ void long_tape_close(const uint32_t* slot, uint32_t columns) {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (threadIdx.x < 32)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(*slot),
+                     "r"(columns));
+}
+
+// Four columns of every lane's row; all lanes of the warp together.
+__device__ __forceinline__ void tmem_put4(uint32_t at, float a, float b, float c, float d) {
+    __syncwarp();
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at),
+                 "r"(__float_as_uint(a)), "r"(__float_as_uint(b)), "r"(__float_as_uint(c)),
+                 "r"(__float_as_uint(d))
+                 : "memory");
+}
+
+__device__ __forceinline__ void tmem_put_done() {
+    __syncwarp();
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_get4(uint32_t at, float& a, float& b, float& c, float& d) {
+    uint32_t u[4];
+    __syncwarp();
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3])
+                 : "r"(at));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    a = __uint_as_float(u[0]);
+    b = __uint_as_float(u[1]);
+    c = __uint_as_float(u[2]);
+    d = __uint_as_float(u[3]);
+}
 
 // Launch shape of a kernel with a per-thread tape in dynamic shared memory
 // (opting in above 48 KB): a grid of the blocks that fit on the GPU at once
@@ -194,6 +276,37 @@ cg_status adj_launch_shape(Kernel kernel, unsigned block, size_t smem, uint64_t 
     CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, (int)block, smem));
     *grid = grid_for(n, block, (unsigned)(per_sm > 0 ? per_sm : 1));
     return CG_OK;
+}
+
+// The same for a kernel with the long tape.  (The occupancy query counts one
+// block per SM for any kernel that allocates tensor memory: measured, 7 run.)
+template <class Kernel>
+cg_status long_launch_shape(Kernel kernel, uint32_t max_iters, uint64_t n, size_t* smem,
+                            unsigned* grid) {
+    *smem = long_tape_bytes(max_iters);
+    if (*smem > 47 * 1024)
+        CG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)*smem));
+    *grid = grid_for(n, ADJ_BLOCK, LONG_WAVES * (unsigned)(228u * 1024u / (*smem + 1024u)));
+    return CG_OK;
+}
+
+// out[N b + k] = block b's sum of acc[k], in a fixed order.
+template <int N>
+__device__ __forceinline__ void block_sums(const double (&acc)[N], double* __restrict__ out) {
+    __shared__ double sums[ADJ_BLOCK / 32][N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        double v = acc[k];
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, o);
+        if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5][k] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < N) {
+        double v = 0.0;
+        for (unsigned w = 0; w < ADJ_BLOCK / 32; ++w) v += sums[w][threadIdx.x];
+        out[(size_t)blockIdx.x * N + threadIdx.x] = v;
+    }
 }
 
 // Backward through one recorded step (the step formulas at the top of this
@@ -337,48 +450,56 @@ __device__ __forceinline__ void polar_de_grad(const ShapeDev& s, const float* __
     grad_outputs(s, dm, px, py, pz, de, zbx, zby, zbz, qbx, qby, qbz, Pb, out);
 }
 
-// polar_de_grad over the long tape (long_tape_bytes(s.max_iters, blockDim.x)
-// bytes at `tape`): the same operations and the same records, each formed
-// once.
+// polar_de_grad over the long tape: the same operations and the same records,
+// each formed once.  All 32 lanes of a warp call it (`valid`: the lane has a
+// point) and go through the steps together, since tensor memory is read and
+// written by whole warps; a lane that has ended writes columns it never reads.
 __device__ __forceinline__ void polar_de_grad_long(const ShapeDev& s, const float* __restrict__ dm,
-                                                   float px, float py, float pz,
-                                                   float* __restrict__ tape, float* out) {
+                                                   bool valid, float px, float py, float pz,
+                                                   const LongTape& tape, float* out) {
     float qx, qy, qz;
     rotate_point(s, px, py, pz, qx, qy, qz);
     const float P = s.power_f;
-    const uint32_t N = s.max_iters, n = blockDim.x;
-    tape += threadIdx.x;
+    const uint32_t N = s.max_iters;
+    constexpr uint32_t n = ADJ_BLOCK;
     float x = qx, y = qy, z = qz, dr = 1.0f, r = 0.0f;
     uint32_t K = 0;
-    bool escaped = false;
-    float* b = tape;
-    for (;;) {
-        float c;
-        if (!polar_radius(s, magnitude2(x, y, z), z, r, c)) {
-            escaped = true;
-            break;
+    bool escaped = false, live = valid;
+    for (uint32_t k = 0; k < N; ++k) {
+        float zr = 0.0f, sn = 0.0f, cs = 0.0f, sp = 0.0f, cp = 0.0f;
+        if (live) {
+            float c;
+            float* b = tape.smem + k * (LONG_FIELDS * n);
+            if (!polar_radius(s, magnitude2(x, y, z), z, r, c)) {
+                escaped = true;
+                live = false;
+            } else {
+                const float t1 = powf(r, __fsub_rn(P, 1.0f));
+                b[0] = dr;
+                b[n] = t1;
+                dr = __fadd_rn(__fmul_rn(__fmul_rn(t1, P), dr), 1.0f);
+                ++K;
+                live = k + 1 < N;
+            }
+            if (live) {
+                const float theta = acosf(c), phi = atan2f(y, x);
+                zr = powf(r, P);
+                sincosf(__fmul_rn(theta, P), &sn, &cs);
+                sincosf(__fmul_rn(phi, P), &sp, &cp);
+                b[2 * n] = theta;
+                b[3 * n] = phi;
+                b[4 * n] = zr;
+            }
         }
-        const float t1 = powf(r, __fsub_rn(P, 1.0f));
-        b[0] = dr;
-        b[n] = t1;
-        dr = __fadd_rn(__fmul_rn(__fmul_rn(t1, P), dr), 1.0f);
-        if (++K == N) break;
-        const float theta = acosf(c), phi = atan2f(y, x), zr = powf(r, P);
-        float sn, cs, sp, cp;
-        sincosf(__fmul_rn(theta, P), &sn, &cs);
-        sincosf(__fmul_rn(phi, P), &sp, &cp);
-        b[2 * n] = theta;
-        b[3 * n] = phi;
-        b[4 * n] = zr;
-        b[5 * n] = sn;
-        b[6 * n] = cs;
-        b[7 * n] = sp;
-        b[8 * n] = cp;
-        b += LONG_FIELDS * n;
-        x = __fadd_rn(__fmul_rn(zr, __fmul_rn(sn, cp)), qx);
-        y = __fadd_rn(__fmul_rn(zr, __fmul_rn(sp, sn)), qy);
-        z = __fadd_rn(__fmul_rn(zr, cs), qz);
+        if (!__any_sync(0xFFFFFFFFu, live)) break;
+        tmem_put4(tape.tmem + 4 * k, sn, cs, sp, cp);
+        if (live) {
+            x = __fadd_rn(__fmul_rn(zr, __fmul_rn(sn, cp)), qx);
+            y = __fadd_rn(__fmul_rn(zr, __fmul_rn(sp, sn)), qy);
+            z = __fadd_rn(__fmul_rn(zr, cs), qz);
+        }
     }
+    tmem_put_done();
     const float ln_r = logf(r);
     const float de = __fdiv_rn(__fmul_rn(0.5f, __fmul_rn(ln_r, r)), dr);
     float r_seed = 0.5f * (ln_r + 1.0f) / dr;
@@ -392,42 +513,35 @@ __device__ __forceinline__ void polar_de_grad_long(const ShapeDev& s, const floa
         r_seed = 0.0f;
     }
     float qbx = 0.0f, qby = 0.0f, qbz = 0.0f, Pb = 0.0f;
+    const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, K);
     StepDeriv d = {};
-    if (K > 0 && escaped) {  // else the last step's angles and r^P stay 0
-        b = tape + (size_t)(K - 1) * LONG_FIELDS * n;
-        d.zr = b[4 * n];
-        d.sn = b[5 * n];
-        d.cs = b[6 * n];
-        d.sp = b[7 * n];
-        d.cp = b[8 * n];
-    }
-    for (uint32_t k = K; k-- > 0;) {
-        b = tape + (size_t)k * LONG_FIELDS * n;
-        d.dr = b[0];
-        d.t1 = b[n];
-        const bool stale = !escaped && k + 1 == N;
-        d.theta = stale ? 0.0f : b[2 * n];
-        d.phi = stale ? 0.0f : b[3 * n];
-        float zr = 0.0f, sn = 0.0f, cs = 0.0f, sp = 0.0f, cp = 0.0f;
-        if (k > 0) {  // z_k, by the operations that formed it
-            b -= LONG_FIELDS * n;
-            zr = b[4 * n];
-            sn = b[5 * n];
-            cs = b[6 * n];
-            sp = b[7 * n];
-            cp = b[8 * n];
-            d.x = __fadd_rn(__fmul_rn(zr, __fmul_rn(sn, cp)), qx);
-            d.y = __fadd_rn(__fmul_rn(zr, __fmul_rn(sp, sn)), qy);
-            d.z = __fadd_rn(__fmul_rn(zr, cs), qz);
-        } else {
-            d.x = qx;
-            d.y = qy;
-            d.z = qz;
+    // Step top - 1's sines and cosines (a loop's last step has none: 0).
+    if (top > 0 && top < N) tmem_get4(tape.tmem + 4 * (top - 1), d.sn, d.cs, d.sp, d.cp);
+    for (uint32_t k = top; k-- > 0;) {
+        float sn = 0.0f, cs = 0.0f, sp = 0.0f, cp = 0.0f;  // step k - 1's
+        if (k > 0) tmem_get4(tape.tmem + 4 * (k - 1), sn, cs, sp, cp);
+        if (k < K) {
+            const float* b = tape.smem + k * (LONG_FIELDS * n);
+            const bool stale = !escaped && k + 1 == N;
+            d.dr = b[0];
+            d.t1 = b[n];
+            d.theta = stale ? 0.0f : b[2 * n];
+            d.phi = stale ? 0.0f : b[3 * n];
+            d.zr = stale ? 0.0f : b[4 * n];
+            if (k > 0) {  // z_k, by the operations that formed it
+                const float zr = *(b - n);  // r^P of step k - 1
+                d.x = __fadd_rn(__fmul_rn(zr, __fmul_rn(sn, cp)), qx);
+                d.y = __fadd_rn(__fmul_rn(zr, __fmul_rn(sp, sn)), qy);
+                d.z = __fadd_rn(__fmul_rn(zr, cs), qz);
+            } else {
+                d.x = qx;
+                d.y = qy;
+                d.z = qz;
+            }
+            float c;
+            polar_radius(s, magnitude2(d.x, d.y, d.z), d.z, d.r, c);
+            polar_back_step(P, d, stale, r_seed, zbx, zby, zbz, drb, qbx, qby, qbz, Pb);
         }
-        float c;
-        polar_radius(s, magnitude2(d.x, d.y, d.z), d.z, d.r, c);
-        polar_back_step(P, d, stale, r_seed, zbx, zby, zbz, drb, qbx, qby, qbz, Pb);
-        d.zr = zr;
         d.sn = sn;
         d.cs = cs;
         d.sp = sp;

@@ -177,12 +177,12 @@ cg_status launch_points_table(const MeshDims& d, const MeshWork& w, uint32_t* po
 cg_status launch_exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* scratch,
                                 uint32_t* total, cudaStream_t st);
 size_t scan_scratch_words(uint32_t n);
-// params[k] = the sum over nwarps per-warp partials, doubles [4 w + k] at
+// params[k] = the sum over `blocks` per-block partials, doubles [4 b + k] at
 // `partial`, in a fixed order (deterministic parameter gradients).
-cg_status launch_sum_partials4(const float* partial, uint32_t nwarps, float* params,
+cg_status launch_sum_partials4(const float* partial, uint32_t blocks, float* params,
                                cudaStream_t st);
 // The calling thread's scratch buffer (at least `floats` words, 16-byte
-// aligned: per-warp partial sums, a work-queue counter) for work enqueued
+// aligned: per-block partial sums, a work-queue counter) for work enqueued
 // on `st`; release_partials(p, st) after the last launch that uses it.
 cg_status acquire_partials(size_t floats, cudaStream_t st, float** out);
 cg_status release_partials(float* partial, cudaStream_t st);

@@ -18,6 +18,7 @@
 #include "common.cuh"
 #include "kernels.cuh"
 #include "lane_pool.cuh"
+#include "point_io.cuh"
 
 namespace cg {
 
@@ -218,19 +219,28 @@ __global__ void __launch_bounds__(128) k_trace_backward(ShapeDev s, CameraDev c,
                                                         const float* __restrict__ g, float cap,
                                                         double* __restrict__ params) {
     extern __shared__ __align__(16) float4 adj_smem[];
+    __shared__ uint32_t slot;
+    const uint32_t columns = long_tape_columns(s.max_iters);
+    LongTape tape;
+    if constexpr (LONG) tape = long_tape_open(reinterpret_cast<float*>(adj_smem), &slot, columns);
     const uint32_t n = c.width * c.height;
+    const WarpWalk walk = warp_walk();
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float t = depth[i], gi = g[i];
-        if (!(t > 0.0f) || gi == 0.0f) continue;
+    for (uint64_t base = walk.first; base < n; base += walk.stride) {
+        const uint32_t i = (uint32_t)base + (threadIdx.x & 31);
+        const bool in = base + (threadIdx.x & 31) < n;
+        const float t = in ? depth[i] : 0.0f, gi = in ? g[i] : 0.0f;
+        const bool hit = t > 0.0f && gi != 0.0f;
+        if (!__any_sync(0xFFFFFFFFu, hit)) continue;
         float d[3];
         pixel_ray(c, i, d);
         float o[8];
         const float x = c.eye[0] + t * d[0], y = c.eye[1] + t * d[1], z = c.eye[2] + t * d[2];
         if constexpr (LONG)
-            polar_de_grad_long(s, dm.m, x, y, z, reinterpret_cast<float*>(adj_smem), o);
-        else
+            polar_de_grad_long(s, dm.m, hit, x, y, z, tape, o);
+        else if (hit)
             polar_de_grad<ADJ_CK>(s, dm.m, x, y, z, adj_tape(adj_smem, s.max_iters, ADJ_CK), o);
+        if (!hit) continue;
         const float dn = o[1] * d[0] + o[2] * d[1] + o[3] * d[2];
         if (!(fabsf(dn) > 1e-6f)) continue;  // grazing ray: no stable depth derivative
         float dt[4];
@@ -247,14 +257,8 @@ __global__ void __launch_bounds__(128) k_trace_backward(ShapeDev s, CameraDev c,
             if (v == v && fabsf(v) < 1e30f) acc[k] += v;
         }
     }
-    // per-warp partial sums, added up in a fixed order by k_sum_partials4
-    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        double v = acc[k];
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, off);
-        if ((threadIdx.x & 31) == 0) params[4 * w + k] = v;
-    }
+    if constexpr (LONG) long_tape_close(&slot, columns);
+    block_sums(acc, params);  // the blocks' are added up by k_sum_partials4
 }
 
 static CameraDev make_camera(const cg_camera& cam) {
@@ -425,19 +429,17 @@ cg_status cg_trace_backward_capped(const cg_shape* shape, const cg_camera* camer
     cudaStream_t st = (cudaStream_t)stream;
     const uint64_t n = (uint64_t)c.width * c.height;
     const bool lng = shape->max_iters <= ADJ_LONG_MAX;
-    const unsigned B = lng ? ADJ_LONG_BLOCK : ADJ_BLOCK;
-    const size_t smem = lng ? long_tape_bytes(shape->max_iters, B)
-                            : adj_tape_bytes(shape->max_iters, ADJ_CK, B);
+    size_t smem = adj_tape_bytes(shape->max_iters, ADJ_CK, ADJ_BLOCK);
     auto kernel = lng ? k_trace_backward<true> : k_trace_backward<false>;
     unsigned G = 0;
-    CG_TRY(adj_launch_shape(kernel, B, smem, n, &G));
-    const uint32_t nwarps = G * (B / 32);
+    CG_TRY(lng ? long_launch_shape(kernel, shape->max_iters, n, &smem, &G)
+               : adj_launch_shape(kernel, ADJ_BLOCK, smem, n, &G));
     float* partial = nullptr;
-    CG_TRY(acquire_partials((size_t)nwarps * 8, st, &partial));
-    kernel<<<G, B, smem, st>>>(s, c, dm, depth, grad_depth, cap,
+    CG_TRY(acquire_partials((size_t)G * 8, st, &partial));
+    kernel<<<G, ADJ_BLOCK, smem, st>>>(s, c, dm, depth, grad_depth, cap,
                                reinterpret_cast<double*>(partial));
     cg_status rs = cuda_status(cudaGetLastError(), "k_trace_backward", __FILE__, __LINE__);
-    if (rs == CG_OK) rs = launch_sum_partials4(partial, nwarps, grad_params, st);
+    if (rs == CG_OK) rs = launch_sum_partials4(partial, G, grad_params, st);
     const cg_status rr = release_partials(partial, st);
     return rs == CG_OK ? rr : rs;
 }

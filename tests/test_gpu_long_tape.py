@@ -54,3 +54,29 @@ def test_batch_product_matches_points(cg, n, iters):
     total, size = terms.sum(0), terms.abs().sum(0)
     got = torch.cat([gpow[None], grot]).double().cuda()
     assert ((got - total).abs() <= (n + 64) * 2.0 ** -24 * size + 1e-30).all()
+
+
+@pytest.mark.parametrize("iters", [9, 10, 17, 18])
+@pytest.mark.parametrize("n", [1, 127, 129, 700001])
+def test_tensor_memory_columns(cg, n, iters):
+    """Where the columns per block change (9, 17 steps), at the edges of a block
+    and with more groups than resident warps, on two streams at once."""
+    import torch
+    from cantucci_gb300 import _ffi
+    from cantucci_gb300.autograd import de_grad
+    lib = _ffi.load()
+    p = torch.as_tensor(W.uniform_points(n, seed=11)).cuda()
+    torch.cuda.synchronize()
+    got = []
+    for stream in (torch.cuda.Stream(), torch.cuda.Stream()):
+        with torch.cuda.stream(stream):
+            got.append(de_grad(p, 7.6, (0.2, -0.1, 0.3), max_iters=iters))
+    torch.cuda.synchronize()
+    _ffi.check(lib.cg_set_option(b"adjoint_ck", 4))
+    try:
+        ref = de_grad(p, 7.6, (0.2, -0.1, 0.3), max_iters=iters)
+    finally:
+        lib.cg_set_option(b"adjoint_ck", 5)
+    for a in got:
+        assert torch.equal(torch.isnan(a), torch.isnan(ref))
+        assert torch.equal(a.nan_to_num(1e9), ref.nan_to_num(1e9))
