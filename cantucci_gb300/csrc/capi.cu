@@ -226,6 +226,7 @@ PlaceOptions place_options(cg_mesher* m) {
     o.numerics = m->numerics;
     o.edge_rows = &m->edge_rows;
     o.edge_data = &m->edge_data;
+    o.edge_total = &m->hcnt->edges;
     return o;
 }
 

@@ -123,8 +123,8 @@ cg_status grow_scratch(DeviceScratch* b, size_t bytes);
 // dual-contouring minimiser of the crossings' tangent planes.
 // With qef the crossings go into an edge table first (one crossing and
 // gradient per sign-changing edge, shared by the edge's cells): its per-row
-// part lives in edge_rows, its per-edge part in edge_data; both are
-// required with qef.
+// part lives in edge_rows, its per-edge part in edge_data; both and
+// edge_total are required with qef.
 struct PlaceOptions {
     bool analytic_normals = false;
     uint32_t root_iters = 0;
@@ -133,6 +133,7 @@ struct PlaceOptions {
     const PlaceParams* pp_dev = nullptr;    // placement parameters in device memory (graphs)
     DeviceScratch* edge_rows = nullptr;
     DeviceScratch* edge_data = nullptr;
+    uint32_t* edge_total = nullptr;  // pinned: the edge table's size on the host
 };
 
 // Steps 2 and 3 of naive_surface_nets on a filled `dists` grid (and, with
@@ -140,6 +141,7 @@ struct PlaceOptions {
 // their capacity; counts land in w.counters.
 // A second stream and a fork / join event pair: with it the quad indices
 // are built concurrently with the vertex placement.
+// (Required with qef.)
 // `timing` / `timing_fork`: where a captured graph records its timing events
 // (record_event).
 struct SideStream {

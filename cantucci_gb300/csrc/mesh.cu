@@ -101,10 +101,7 @@ __global__ void __launch_bounds__(256) k_cells(const uint32_t* __restrict__ sgn,
                                                uint32_t* __restrict__ wordoff,
                                                uint32_t* __restrict__ rowcnt,
                                                MeshCounters* __restrict__ cnt) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        cnt->status = 0;
-        cnt->edges = 0;
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) cnt->status = 0;
     const uint32_t rows = d.res * d.res;
     [[maybe_unused]] const uint64_t nc = (uint64_t)rows * d.Wc;
     const RowLanes g(d);
@@ -217,7 +214,6 @@ __global__ void __cluster_dims__(kRowsCluster, 1, 1) __launch_bounds__(512)
         cnt->vertices = all.x;
         cnt->quads = all.y;
         cnt->status = 0;
-        cnt->edges = 0;
     }
 }
 
@@ -225,14 +221,15 @@ __global__ void __cluster_dims__(kRowsCluster, 1, 1) __launch_bounds__(512)
 // vertices and stores them through shared memory as 16-byte chunks (32
 // vertices = 896 bytes = 56 float4), so the stores are coalesced whether
 // `verts` is device memory or pinned host memory written over the C2C link.
+// Dual contouring is short of warps to hide its table's loads and its serial
+// rotations behind: six blocks per SM with a few spilled words take 213 ->
+// 193 us at 256^3 cells (five: 703, six: 692, seven: 693, four: 712 per mesh).
 template <int M, bool AN, bool ROOT, bool QEF>
-__global__ void __launch_bounds__(128, (AN || QEF) ? 5 : (ROOT ? 1 : 9)) k_place(ShapeDev s, PlaceParams pp, MeshDims d,
-                                               const float* __restrict__ dists,
-                                               const uint32_t* __restrict__ cellidx,
-                                               MeshCounters* __restrict__ cnt,
-                                               cg_vertex* __restrict__ verts, uint64_t vcap,
-                                               uint32_t root_iters, EdgeTable et,
-                                               const PlaceParams* __restrict__ ppp) {
+__global__ void __launch_bounds__(128, QEF ? 6 : AN ? 5 : ROOT ? 1 : 9) k_place(
+    ShapeDev s, PlaceParams pp, MeshDims d, const float* __restrict__ dists,
+    const uint32_t* __restrict__ cellidx, MeshCounters* __restrict__ cnt,
+    cg_vertex* __restrict__ verts, uint64_t vcap, uint32_t root_iters, EdgeTable et,
+    const PlaceParams* __restrict__ ppp) {
     if (ppp) pp = *ppp;
     __shared__ __align__(16) float stage[4][32 * 7];
     const uint32_t V = cnt->vertices;
@@ -655,7 +652,7 @@ cg_status grow_scratch(DeviceScratch* b, size_t bytes) {
 // in w.counters->edges.
 static cg_status launch_edge_rows(const MeshDims& d, const MeshWork& w, const PlaceOptions& opt,
                                   cudaStream_t st) {
-    if (!opt.edge_rows || !opt.edge_data) {
+    if (!opt.edge_rows || !opt.edge_data || !opt.edge_total) {
         set_error("dual contouring needs edge scratch buffers");
         return CG_EINVAL;
     }
@@ -829,32 +826,43 @@ cg_status launch_mesh_from_dists(const ShapeDev& s, const SpanSetup& su, const M
                                  uint32_t* idx, uint64_t icap, cudaStream_t st,
                                  cudaEvent_t ev_after_vertices, bool signs_ready,
                                  const PlaceOptions& opt, const SideStream* side) {
-    CG_TRY(launch_cells(d, w, st, signs_ready));
-    // Dual contouring: the edge table (its size is read back once).
-    auto edge_table = [&](EdgeTable* et) -> cg_status {
-        CG_TRY(launch_edge_rows(d, w, opt, st));
-        uint32_t E = 0;
-        CG_CUDA(cudaMemcpyAsync(&E, &w.counters->edges, sizeof E, cudaMemcpyDeviceToHost, st));
-        CG_CUDA(cudaStreamSynchronize(st));
-        return launch_edge_data(s, place_params(su), d, w, opt, E, st, et);
-    };
     EdgeTable et{};
     if (side) {
+        // Dual contouring: the edge table, whose size is read back once.  Its
+        // counts go first (signs_ready), so that they reach the host on the
+        // side stream while the cells and the vertex list are made (256^3
+        // cells: 692 -> 686 us, the counts after the list and waited for on
+        // `st` before).
+        if (opt.qef) {
+            CG_TRY(launch_edge_rows(d, w, opt, st));
+            CG_CUDA(cudaEventRecord(side->fork, st));
+            CG_CUDA(cudaStreamWaitEvent(side->stream, side->fork, 0));
+            CG_CUDA(cudaMemcpyAsync(opt.edge_total, &w.counters->edges, sizeof(uint32_t),
+                                    cudaMemcpyDeviceToHost, side->stream));
+        }
+        CG_TRY(launch_cells(d, w, st, signs_ready));
+        CG_CUDA(cudaEventRecord(side->fork, st));
+        if (opt.qef) {
+            CG_CUDA(cudaStreamSynchronize(side->stream));
+            CG_TRY(launch_edge_data(s, place_params(su), d, w, opt, *opt.edge_total, st, &et));
+        }
         // The quads need only the cell table and the signs: they run on the
         // side stream while the (compute-bound) vertex placement runs here.
-        CG_CUDA(cudaEventRecord(side->fork, st));
         CG_CUDA(cudaStreamWaitEvent(side->stream, side->fork, 0));
         CG_TRY(launch_quad_count(d, w, side->stream));
         CG_TRY(launch_quad_emit(d, w, idx, icap, side->stream));
         CG_CUDA(cudaEventRecord(side->join, side->stream));
-        if (opt.qef) CG_TRY(edge_table(&et));
         CG_TRY(launch_place(s, su, d, w, verts, vcap, st, opt, et));
         if (ev_after_vertices)
             CG_CUDA(record_event(ev_after_vertices, st, side->timing, side->timing_fork));
         CG_CUDA(cudaStreamWaitEvent(st, side->join, 0));
         return CG_OK;
     }
-    if (opt.qef) CG_TRY(edge_table(&et));
+    if (opt.qef) {
+        set_error("dual contouring needs the side stream");
+        return CG_EINVAL;
+    }
+    CG_TRY(launch_cells(d, w, st, signs_ready));
     CG_TRY(launch_place(s, su, d, w, verts, vcap, st, opt, et));
     if (ev_after_vertices) CG_CUDA(record_event(ev_after_vertices, st));
     CG_TRY(launch_quad_count(d, w, st));

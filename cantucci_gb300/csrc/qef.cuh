@@ -263,7 +263,8 @@ __device__ __forceinline__ void qef_solve(const Qef& q, float hx, float hy, floa
         const float r1 = q.b1 - (q.a01 * cx + q.a11 * cy + q.a12 * cz);
         const float r2 = q.b2 - (q.a02 * cx + q.a12 * cy + q.a22 * cz);
         float v[3][3] = {{1.0f, 0.0f, 0.0f}, {0.0f, 1.0f, 0.0f}, {0.0f, 0.0f, 1.0f}};
-#pragma unroll
+        // Rolled: one sweep is in the instruction cache with the gradient's loop.
+#pragma unroll 1
         for (int sweep = 0; sweep < 5; ++sweep) {
             jacobi_rotate<0, 1>(a, v);
             jacobi_rotate<0, 2>(a, v);
