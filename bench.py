@@ -37,7 +37,7 @@ WORKLOAD = ("single octree span, 512^3 cells / 513^3 = 135,005,697 corners, Mand
 FLOPS_PER_STEP = 76   # P=8 iteration: magnitude, dr, polynomial, + p (each op = 1 flop)
 FLOPS_PER_ESCAPE = 6  # the final magnitude of an escaping point
 FLOPS_PER_POINT = 4   # ln(r) * r, * 0.5, / dr
-LAUNCHES_PER_MESH = 12  # k_de_grid_brick (sign words fused), k_cells, 3x scan, k_vertex_list,
+LAUNCHES_PER_MESH = 12  # k_de_grid_units (sign words fused), k_cells, 3x scan, k_vertex_list,
 #                         k_place, k_quad_count, 3x scan, k_quad_emit (ncu launch list: 12 per mesh)
 
 
@@ -374,10 +374,10 @@ def extra_normals(dev, n=16 << 20, cpu=True):
            "tangent_all_vs_fd6_speedup": ms_fd / ms_tan4,
            "fwd_tangent_fast_normals_pts_per_s": n / (ms_tanf * 1e-3),
            "tangent_fast_normals_vs_fd6_speedup": ms_fd / ms_tanf,
-           "modes": "adjoint = reverse mode with checkpoint recompute (DE, grad, d/dpower, "
-                    "d/drotation; checkpoint every 5 steps, tape in shared memory); "
-                    "adjoint_fast_recompute = the same with each segment recomputed from its "
-                    "exact checkpoint in the fast polar arithmetic (cg_set_option "
+           "modes": "adjoint = reverse mode (DE, grad, d/dpower, d/drotation; every step's "
+                    "record in shared and tensor memory); "
+                    "adjoint_fast_recompute = checkpoints every 5 steps, each segment "
+                    "recomputed from its exact checkpoint in the fast polar arithmetic (cg_set_option "
                     "adjoint_recompute 1); tangent_normals = forward mode along x, y, z (DE, "
                     "grad, d/drotation); tangent_all = forward mode with the power direction too"}
     if not cpu:
@@ -1007,7 +1007,7 @@ def run_ours(args, rank, world, local_rank):
     peak2_tf = fp32_peak(True) / 1e12
     roofline = {
         "bound": "fp32",
-        "kernel": {0: "k_de_grid_brick", 1: "k_de_grid", 2: "k_de_grid_brick",
+        "kernel": {0: "k_de_grid_units", 1: "k_de_grid", 2: "k_de_grid_brick",
                    3: "k_de_grid_p8x2"}[args.de_kernel],
         "achieved": achieved, "peak": peak_tf,
         "unit": "TFLOP/s", "frac": achieved / peak_tf, "traffic": None,

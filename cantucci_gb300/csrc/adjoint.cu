@@ -173,8 +173,8 @@ __global__ void __launch_bounds__(1024) k_sum_partials4(const double* __restrict
 // derivatives) in double, added up in a fixed order by k_surface_l1_sum.  One
 // pass over the points in place of the gradients of all of them, a dozen
 // reductions and selections on those and the synchronisations that selecting
-// by a mask takes: 592 -> 75 us per call for 125 K points, 44 us of either in
-// the sweep.  MODE 0: long tape, 1: checkpoints, 2: fast recompute.
+// by a mask takes: 592 -> 96 us per call from Python for 125 K points, 35 us of
+// it the sweep.  MODE 0: long tape, 1: checkpoints, 2: fast recompute.
 template <int MODE>
 __global__ void __launch_bounds__(128) k_surface_l1(ShapeDev s, Dm3 dm,
                                                     const float* __restrict__ pts, uint64_t n,

@@ -150,9 +150,9 @@ __global__ void __launch_bounds__(256) k_vertex_list(MeshDims d, const uint32_t*
 // through distributed shared memory) gives every word's first vertex id and,
 // beside it, every row's first quad.  Latency-bound either way; six launches
 // became one (a res-64 leaf's mesh 71 -> 62 us with the timing events off the
-// path).
+// path; 5.8 us of it this kernel).
 constexpr uint32_t kClusterRowsMaxRes = 64;
-// (16 CTAs: a cluster of 8 with 1024 threads each took 9.5 us, this 7.)
+// (16 CTAs: a cluster of 8 with 1024 threads each took 2.5 us more.)
 constexpr unsigned kRowsCluster = 16;
 
 __global__ void __cluster_dims__(kRowsCluster, 1, 1) __launch_bounds__(512)
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(128, QEF ? 6 : AN ? 5 : ROOT ? 1 : 9) k_place(
 // vertices in the span a warp takes 4 (28 samples, one round: the shortest
 // chain); from kSpreadTwoRounds on it takes 9 (63 samples, two rounds), which
 // shares the twelve crossings of a cell's edges among more samples and leaves
-// one lane idle in 64 (a res-64 leaf of 30 K vertices: 23.5 -> 17 us against
+// one lane idle in 64 (a res-64 leaf of 34 K vertices: 23.5 -> 18.9 us against
 // eight lanes per vertex, each forming the position).  The same operations as
 // k_place<M, false, false, false>, so the same bits.  The loop bound is
 // warp-uniform.

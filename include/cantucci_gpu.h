@@ -485,8 +485,9 @@ cg_status cg_trace_backward_capped(const cg_shape* shape, const cg_camera* camer
  * (kind CG_SHAPE_MANDELBULB_POLAR, src/shape/mandelbulb.frag:1-39, rotated).
  * No reference counterpart: it replaces the six extra estimator calls of the
  * central-difference normal (src/mesh/buffer.rs:256-266) and gives the
- * parameter gradients for fitting.  Iterates are recomputed from
- * checkpoints, never stored.  max_iters <= 64.
+ * parameter gradients for fitting.  Up to 20 iterations every step's
+ * record stays on chip; above, iterates are recomputed from checkpoints.
+ * max_iters <= 64.
  * out: device, n x 8 floats: DE, dDE/dx, dDE/dy, dDE/dz, dDE/dpower,
  * dDE/da, dDE/db, dDE/dc (Euler angles). */
 cg_status cg_de_grad(const cg_shape* shape, const float* points, uint64_t n, float* out,
@@ -536,13 +537,16 @@ cg_status cg_fd_grad(const cg_shape* shape, const float* points, uint64_t n, flo
 
 /* ---- measurement -------------------------------------------------------- */
 
-/* Process-wide tuning knobs.  "de_grid_kernel": 0 auto, 1 one corner per
- * thread in GridTable order, 2 2x4x4 bricks per warp, 3 (P=8 only) one
- * 4x4x4 brick per warp, two corners per thread with packed f32x2 arithmetic.
+/* Process-wide tuning knobs.  "de_grid_kernel": 0 auto (by resolution: one
+ * corner per thread, one core unit per block, bricks, or a queue of core units
+ * and face groups), 1 one corner per thread in GridTable order, 2 2x4x4 bricks
+ * per warp, 3 (P=8 only) one 4x4x4 brick per warp, two corners per thread with
+ * packed f32x2 arithmetic.
  * "place_blocks_per_sm" (1..1024, default 128): the vertex placement's grid.
  * "side_stream_priority" (1 default, or 0): whether meshers created
  * afterwards run their quads and copies on a highest-priority stream.
- * "trace_kernel": 1 work-queue march (default), 0 one pixel per thread.
+ * "trace_kernel": 1 (default) rays of a block in one pool fed from a queue,
+ * 0 one pixel per thread.
  * "mesh_graphs" (1 default, or 0): meshes up to resolution 128 (other than
  * dual contouring) replay a CUDA graph the mesher captured for that
  * resolution, shape and option set, the span going in as a parameter block.
