@@ -25,8 +25,9 @@ __global__ void __launch_bounds__(256) k_de_points(ShapeDev s, const float* __re
     }
 }
 
-// Large batches: each warp takes its points through a lane pool.
-template <int M>
+// Large batches: each warp takes its points through a lane pool.  MU: the mode
+// of points taken whole.
+template <int M, int MU>
 struct PointTask {
     const ShapeDev& s;
     const float* __restrict__ pts;
@@ -38,25 +39,22 @@ struct PointTask {
     __device__ __forceinline__ bool step() { return de.step(s); }
     __device__ __forceinline__ void finish(uint64_t i) { out[i] = de.value(s); }
     __device__ __forceinline__ uint32_t steps() const { return de.it; }
+    __device__ __forceinline__ void whole(uint64_t i) {
+        out[i] = eval<MU>(s, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]);
+    }
 };
 
 // Lanes that wait in a pool: more where a step is short.
 template <int M>
-constexpr int kPointFlush = M == MODE_P8 || M == MODE_P8_FAST ? 12 : 8;
+constexpr int kPointFlush = M == MODE_P8 ? 12 : 8;
 
-// MU: the mode of the loop for points side by side.
 template <int M, int MU>
 __global__ void __launch_bounds__(128) k_de_points_pool(ShapeDev s, const float* __restrict__ pts,
                                                         uint64_t n, float* __restrict__ out) {
     const WarpWalk w = warp_walk();
     if (w.first >= n) return;
-    if (points_side_by_side(pts, w, n)) {
-        for (uint64_t i = w.first + (threadIdx.x & 31); i < n; i += w.stride)
-            out[i] = eval<MU>(s, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]);
-        return;
-    }
-    PointTask<M> task{s, pts, out, {}};
-    warp_pool(w, n, kPointFlush<M>, s.max_iters, task);
+    PointTask<M, MU> task{s, pts, out, {}};
+    warp_pool(w, n, points_side_by_side(pts, w, n) ? 32 : kPointFlush<M>, s.max_iters, task);
 }
 
 // Corner (x, y, z) of a span grid: p = start + across * (v / res)
@@ -348,23 +346,24 @@ static bool launch_points_pool(const ShapeDev& s, const float* pts, uint64_t n, 
     return G != 0;
 }
 
-// True if the batch is large enough for a pool kernel (and was launched).
+// True if the batch is large enough for a pool kernel (and was launched).  The
+// exact estimators only: a step of the fast ones is too short for it (9 M points
+// on the surface 4 to 8 % slower, 3 M points anywhere no faster).
+// In us, the plain kernel -> the pool: polar power 8,
+// 3 M uniform points 396 -> 236, 16 M 2082 -> 1080; 3 M on the surface 396 ->
+// 403, 16 M 2082 -> 2050; 9 M of a grid 510 -> 515; Mandelbulb<8>, 3 M uniform
+// 136 -> 109, on the surface 136 -> 126, a grid 74 -> 60; 1.7 M polar uniform
+// 225 -> 155, on the surface 225 -> 237.
 static bool launch_points_pool_mode(const ShapeDev& s, const float* pts, uint64_t n, float* out,
                                     uint32_t numerics, cudaStream_t st) {
-    if (n < (1u << 18) || s.max_iters < 1) return false;
+    if (s.max_iters < 1) return false;
     switch (mode_of(s, numerics)) {
-    case MODE_SPHERE: return false;
     case MODE_P8:
         return p8_unrolled(s) ? launch_points_pool<MODE_P8, MODE_P8_IT15>(s, pts, n, out, st)
                               : launch_points_pool<MODE_P8>(s, pts, n, out, st);
     case MODE_INT: return launch_points_pool<MODE_INT>(s, pts, n, out, st);
     case MODE_POLAR: return launch_points_pool<MODE_POLAR>(s, pts, n, out, st);
-    case MODE_INT_POLY: return launch_points_pool<MODE_INT_POLY>(s, pts, n, out, st);
-    case MODE_POLAR_FAST: return launch_points_pool<MODE_POLAR_FAST>(s, pts, n, out, st);
-    default:
-        return p8_unrolled(s)
-                   ? launch_points_pool<MODE_P8_FAST, MODE_P8_FAST_IT15>(s, pts, n, out, st)
-                   : launch_points_pool<MODE_P8_FAST>(s, pts, n, out, st);
+    default: return false;
     }
 }
 

@@ -95,12 +95,15 @@ __device__ __forceinline__ bool points_side_by_side(const float* __restrict__ pt
 // 32 lanes.
 //   task.start(i)   begin point i            task.step()  one step, false at the end
 //   task.finish(i)  write point i's result   task.steps() the steps of the point
+//   task.whole(i)   all of point i
 // `wait`: the lanes that wait before results are written and new points taken
-// together; 32 keeps the lanes in step, group by group.  Lanes in step also
-// agree on the branches inside the trigonometric functions, so where steps are
-// alike the pool costs 15 to 25 %.  Points side by side are the caller's to
-// tell; points that run most of `max_steps` (on the surface) show here: once a
-// warp's worth of points has averaged 0.45 of it, the lanes stay in step.
+// together.  Lanes in step also agree on the branches inside the trigonometric
+// functions, so where steps are alike the pool costs 15 to 25 %: there the
+// points are taken whole, group by group.  Points side by side are the caller's
+// to tell (wait 32); points that run most of `max_steps` (on the surface) show
+// here: if fewer than `wait` of the first 32 have ended after a fifth of it (of
+// uniform points in the cube 73 % have after two of 15 steps, of points on the
+// surface 4 % after three), or a warp's worth of points has averaged 0.45 of it.
 template <class Task>
 __device__ __forceinline__ void warp_pool(const WarpWalk& w, uint64_t n, int wait,
                                           uint32_t max_steps, Task& task) {
@@ -111,18 +114,24 @@ __device__ __forceinline__ void warp_pool(const WarpWalk& w, uint64_t n, int wai
     const uint64_t count = (groups - 1) * 32 + (last < 32 ? last : 32);
     uint64_t next = 0, mine = 0;
     uint32_t ended = 0, steps = 0;
+    const bool alike = wait == 32;
+    uint32_t probe = max(max_steps / 5, 1u);
     bool have = false, busy = false;
-    for (;;) {
+    while (wait < 32 || next > 0) {
         const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !busy);
         const uint32_t done = __ballot_sync(0xFFFFFFFFu, have && !busy);
         // Enough lanes wait for new points or, when there are none, with results.
         const uint32_t waiting = next < count ? idle : done;
         if (__popc(waiting) >= wait || idle == 0xFFFFFFFFu) {
             if (have && !busy) task.finish(mine);
-            if (wait < 32) {
-                ended += __popc(done);
-                steps += __reduce_add_sync(0xFFFFFFFFu, have && !busy ? task.steps() : 0u);
-                if (ended >= 32 && (float)steps > 0.45f * (float)ended * (float)max_steps) wait = 32;
+            if (wait == 32) break;  // every lane has ended
+            ended += __popc(done);
+            steps += __reduce_add_sync(0xFFFFFFFFu, have && !busy ? task.steps() : 0u);
+            if (ended >= 32 && (float)steps > 0.45f * (float)ended * (float)max_steps) {
+                wait = 32;
+                have = have && busy;
+                if (!__any_sync(0xFFFFFFFFu, busy)) break;
+                continue;
             }
             if (!busy) {
                 const uint64_t k = next + __popc(idle & below);
@@ -134,14 +143,27 @@ __device__ __forceinline__ void warp_pool(const WarpWalk& w, uint64_t n, int wai
             if (!__any_sync(0xFFFFFFFFu, busy)) break;
         }
         if (busy) busy = task.step();
+        if (--probe == 0 && next == 32) wait = 32;
+    }
+    // A grid's rows and a stride near a multiple of them would leave each warp
+    // one part of the shape: the warps change places from group to group.
+    const uint64_t turn = alike ? (w.stride * 618 / 1000) & ~31ull : 0;
+    const uint64_t end = alike ? (n + w.stride - 1) / w.stride * 32 : count;
+    for (uint64_t first = w.first; next < end; next += 32) {
+        const uint64_t k = next + (threadIdx.x & 31), i = first + (k >> 5) * w.stride + (k & 31);
+        if (i < n) task.whole(i);
+        first += turn;
+        if (first >= w.stride) first -= w.stride;
     }
 }
 
-// The blocks (of 128 threads) of a pool kernel over n points: four points to a
-// lane, and for larger batches up to twice the blocks that fit on the GPU at
-// once (blocks then end at different times and the SMs stay full: 209 against
-// 253 us for 3M points of a grid).  0 when four points to a lane do not fill
-// the GPU, where a pool gains less than the missing warps cost.
+// The blocks (of 128 threads) of a pool kernel over n points: 16 points to a
+// lane, between two and eight times the blocks that fit on the GPU at once
+// (blocks then end at different times and the SMs stay full: 209 against 253 us
+// for 3 M points of a grid at two, 868 against 805 for 16 M at five).  0 with
+// fewer than 8 points to a lane of the blocks that fit, where a pool gains less
+// than its uneven end costs (1 M points: uniform 135 -> 101 us, but on the
+// surface 135 -> 147 and of a grid 80 -> 92).
 template <class Kernel>
 unsigned pool_grid(Kernel kernel, uint64_t n) {
     static int per_sm = 0;
@@ -152,8 +174,10 @@ unsigned pool_grid(Kernel kernel, uint64_t n) {
             b = 1;
         per_sm = b;
     }
-    const unsigned g = grid_for((n + 3) / 4, 128, 2 * per_sm);
-    return g >= (unsigned)(sm_count() * per_sm) ? g : 0;
+    const uint64_t lanes = (uint64_t)sm_count() * per_sm * 128;
+    if (n < 8 * lanes) return 0;
+    const uint64_t resident = lanes / 128, even = n / (16 * 128);
+    return (unsigned)std::min(std::max(even, 2 * resident), 8 * resident);
 }
 
 }  // namespace cg

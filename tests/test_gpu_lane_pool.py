@@ -43,7 +43,9 @@ def points(order, n, shape):
 
 @pytest.mark.parametrize("order,n", [("random", 1_500_000), ("random", 1_500_031),
                                      ("side_by_side", 1_500_017), ("surface", 1_500_001),
-                                     ("special", 1_500_007), ("random", 4_000_003)])
+                                     ("special", 1_500_007), ("random", 4_000_003),
+                                     ("side_by_side", 2_500_017), ("surface", 2_500_001),
+                                     ("special", 2_500_007)])
 @pytest.mark.parametrize("name", ["p8", "p8_it9", "int6", "polar", "p8_fast", "int6_fast",
                                   "polar_fast", "one_step", "sphere"])
 def test_large_batch_same_bits(cg, name, order, n):
