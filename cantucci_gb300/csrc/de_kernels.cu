@@ -488,8 +488,10 @@ static cg_status launch_grid_mode(const ShapeDev& s, const GridDev& g, float* ou
         const uint64_t units8 = rows * ((bz + 7) / 8);
         if (units8 >= 4ull * sm_count() * 8 * (B / 32)) {
             const uint64_t units = core_units(shift) + (face_items(shift) + 7) / 8;
-            uint32_t* queue = sgn ? sgn + words : nullptr;
-            CG_TRY(clear(queue, 1));
+            // (A sphere's units are so short that they would wait for the queue:
+            // a mesh of 256^3 cells 195 us with it, 155 without.)
+            uint32_t* queue = sgn && M != MODE_SPHERE ? sgn + words : nullptr;
+            if (queue) CG_TRY(clear(queue, 1));
             k_de_grid_units<M><<<grid_for(units * 32, B, 8), B, 0, st>>>(s, g, out, sgn, W, shift,
                                                                          queue, gp);
         } else {
