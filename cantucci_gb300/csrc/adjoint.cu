@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(128) k_de_grad(ShapeDev s, Dm3 dm, const float
     }
 }
 
-// The same over the long tape (max_iters <= ADJ_LONG_MAX).
+// The same over the long tape (takes_long_tape).
 __global__ void __launch_bounds__(ADJ_BLOCK, LONG_BLOCKS) k_de_grad_long(ShapeDev s, Dm3 dm,
                                                             const float* __restrict__ pts,
                                                             uint64_t n, float* __restrict__ out) {
@@ -111,25 +111,28 @@ __global__ void __launch_bounds__(128) k_de_spatial_grad(ShapeDev s, const float
 template <bool LONG>
 __global__ void __launch_bounds__(128) k_de_vjp(ShapeDev s, Dm3 dm, const float* __restrict__ pts,
                                                 const float* __restrict__ g, uint64_t n,
-                                                float* __restrict__ gp, double* __restrict__ params) {
+                                                float* __restrict__ gp, double* __restrict__ params,
+                                                float* __restrict__ whole) {
     extern __shared__ __align__(16) float4 adj_smem[];
     __shared__ uint32_t slot;
     const uint32_t columns = long_tape_columns(s.max_iters);
     LongTape tape;
     if constexpr (LONG) tape = long_tape_open(reinterpret_cast<float*>(adj_smem), &slot, columns);
     const WarpWalk walk = warp_walk();
+    const uint32_t lane = threadIdx.x & 31;
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (uint64_t base = walk.first; base < n; base += walk.stride) {
-        const uint64_t i = base + (threadIdx.x & 31);
-        const bool in = i < n;
-        const float* p = pts + 3 * (in ? i : base);
+    // (LONG: a warp's lanes stay together to the end)
+    for (uint64_t i = walk.first + lane; LONG ? i - lane < n : i < n; i += walk.stride) {
         float o[8];
-        if constexpr (LONG)
+        if constexpr (LONG) {
+            const bool in = i < n;
+            const float* p = pts + 3 * (in ? i : i - lane);
             polar_de_grad_long(s, dm.m, in, p[0], p[1], p[2], tape, o);
-        else if (in)
-            polar_de_grad<ADJ_CK>(s, dm.m, p[0], p[1], p[2],
+            if (!in) continue;
+        } else {
+            polar_de_grad<ADJ_CK>(s, dm.m, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2],
                                   adj_tape(adj_smem, s.max_iters, ADJ_CK), o);
-        if (!in) continue;
+        }
         const float gi = g[i];
         if (gp) {
             gp[3 * i] = gi * o[1];
@@ -145,7 +148,7 @@ __global__ void __launch_bounds__(128) k_de_vjp(ShapeDev s, Dm3 dm, const float*
         }
     }
     if constexpr (LONG) long_tape_close(&slot, columns);
-    if (params) block_sums(acc, params);
+    if (params || whole) block_sums(acc, params, whole);
 }
 
 // params[k] = the sum over blocks b < blocks of partial[4 b + k], in a fixed
@@ -382,7 +385,7 @@ template <int CK, bool FR>
 static cg_status launch_de_grad(const ShapeDev& sd, const Dm3& dm, uint32_t max_iters,
                                 const float* points, uint64_t n, float* out, cudaStream_t st) {
     unsigned G = 0;
-    if (CK == ADJ_CK && !FR && max_iters <= ADJ_LONG_MAX) {
+    if (CK == ADJ_CK && !FR && takes_long_tape(max_iters)) {
         size_t smem = 0;
         CG_TRY(long_launch_shape(k_de_grad_long, max_iters, n, &smem, &G));
         k_de_grad_long<<<G, ADJ_BLOCK, smem, st>>>(sd, dm, points, n, out);
@@ -490,16 +493,19 @@ cg_status cg_de_backward(const cg_shape* shape, const float* points, const float
         if (grad_params) CG_CUDA(cudaMemsetAsync(grad_params, 0, 4 * sizeof(float), st));
         return CG_OK;
     }
-    const bool lng = shape->max_iters <= ADJ_LONG_MAX;
+    const bool lng = takes_long_tape(shape->max_iters);
     size_t smem = adj_tape_bytes(shape->max_iters, ADJ_CK, ADJ_BLOCK);
     auto kernel = lng ? k_de_vjp<true> : k_de_vjp<false>;
     unsigned G = 0;
     CG_TRY(lng ? long_launch_shape(kernel, shape->max_iters, n, &smem, &G)
                : adj_launch_shape(kernel, ADJ_BLOCK, smem, n, &G));
+    // One block writes the sums itself.
     float* partial = nullptr;
-    if (grad_params) CG_TRY(acquire_partials((size_t)G * 8, st, &partial));
+    if (grad_params && G > 1) CG_TRY(acquire_partials((size_t)G * 8, st, &partial));
     kernel<<<G, ADJ_BLOCK, smem, st>>>(make_shape_dev(*shape), rotation_derivatives(*shape), points,
-                               grad_out, n, grad_points, reinterpret_cast<double*>(partial));
+                                       grad_out, n, grad_points,
+                                       reinterpret_cast<double*>(partial),
+                                       G > 1 ? nullptr : grad_params);
     cg_status rs = cuda_status(cudaGetLastError(), "k_de_vjp", __FILE__, __LINE__);
     if (rs == CG_OK && partial) rs = launch_sum_partials4(partial, G, grad_params, st);
     if (partial) {
@@ -516,7 +522,7 @@ cg_status cg_surface_l1(const cg_shape* shape, const float* points, uint64_t n, 
         set_error("NULL buffer");
         return CG_EINVAL;
     }
-    const bool lng = g_adjoint_fastrec == 0 && shape->max_iters <= ADJ_LONG_MAX;
+    const bool lng = g_adjoint_fastrec == 0 && takes_long_tape(shape->max_iters);
     size_t smem = adj_tape_bytes(shape->max_iters, ADJ_CK, ADJ_BLOCK);
     auto kernel = lng ? k_surface_l1<0> : (g_adjoint_fastrec ? k_surface_l1<2> : k_surface_l1<1>);
     cudaStream_t st = (cudaStream_t)stream;

@@ -181,7 +181,16 @@ __device__ __forceinline__ StepDeriv tape_get(const AdjTape& t, uint32_t slot) {
 // with their sums, 1 M points, 285 -> 235; the depth map's backward pass,
 // 512 x 512, 77 -> 64; up to 20 K points the same (latency).
 constexpr int LONG_FIELDS = 5;
-constexpr uint32_t ADJ_LONG_MAX = 20;  // the longest loop that takes it
+// The longest loop that takes it: the last with three blocks per SM (1 M points
+// at 30 steps, checkpoints 779 us, long tape 530; at 21, 571 and 338).
+constexpr uint32_t ADJ_LONG_MAX = 30;
+
+// (Up to ADJ_CK steps the checkpointed tape holds them all too and needs no
+// tensor memory: a 256 x 256 backward pass of 5 steps 21 against 25 us.  At 6
+// steps the long tape is ahead, 1 M points 175 -> 92.)
+__host__ __device__ constexpr bool takes_long_tape(uint32_t max_iters) {
+    return max_iters > (uint32_t)ADJ_CK && max_iters <= ADJ_LONG_MAX;
+}
 
 // Columns for the sines and cosines of max_iters - 1 steps: a power of two.
 __host__ __device__ constexpr uint32_t long_tape_columns(uint32_t max_iters) {
@@ -291,9 +300,11 @@ cg_status long_launch_shape(Kernel kernel, uint32_t max_iters, uint64_t n, size_
     return CG_OK;
 }
 
-// out[N b + k] = block b's sum of acc[k], in a fixed order.
+// out[N b + k] = block b's sum of acc[k], in a fixed order; with `whole` (a grid
+// of one block) whole[k] instead, rounded.
 template <int N>
-__device__ __forceinline__ void block_sums(const double (&acc)[N], double* __restrict__ out) {
+__device__ __forceinline__ void block_sums(const double (&acc)[N], double* __restrict__ out,
+                                           float* __restrict__ whole = nullptr) {
     __shared__ double sums[ADJ_BLOCK / 32][N];
 #pragma unroll
     for (int k = 0; k < N; ++k) {
@@ -305,7 +316,8 @@ __device__ __forceinline__ void block_sums(const double (&acc)[N], double* __res
     if (threadIdx.x < N) {
         double v = 0.0;
         for (unsigned w = 0; w < ADJ_BLOCK / 32; ++w) v += sums[w][threadIdx.x];
-        out[(size_t)blockIdx.x * N + threadIdx.x] = v;
+        if (whole) whole[threadIdx.x] = (float)v;
+        else out[(size_t)blockIdx.x * N + threadIdx.x] = v;
     }
 }
 

@@ -428,7 +428,7 @@ cg_status cg_trace_backward_capped(const cg_shape* shape, const cg_camera* camer
     const Dm3 dm = rotation_derivatives(*shape);
     cudaStream_t st = (cudaStream_t)stream;
     const uint64_t n = (uint64_t)c.width * c.height;
-    const bool lng = shape->max_iters <= ADJ_LONG_MAX;
+    const bool lng = takes_long_tape(shape->max_iters);
     size_t smem = adj_tape_bytes(shape->max_iters, ADJ_CK, ADJ_BLOCK);
     auto kernel = lng ? k_trace_backward<true> : k_trace_backward<false>;
     unsigned G = 0;

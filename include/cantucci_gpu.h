@@ -485,7 +485,7 @@ cg_status cg_trace_backward_capped(const cg_shape* shape, const cg_camera* camer
  * (kind CG_SHAPE_MANDELBULB_POLAR, src/shape/mandelbulb.frag:1-39, rotated).
  * No reference counterpart: it replaces the six extra estimator calls of the
  * central-difference normal (src/mesh/buffer.rs:256-266) and gives the
- * parameter gradients for fitting.  Up to 20 iterations every step's
+ * parameter gradients for fitting.  Up to 30 iterations every step's
  * record stays on chip; above, iterates are recomputed from checkpoints.
  * max_iters <= 64.
  * out: device, n x 8 floats: DE, dDE/dx, dDE/dy, dDE/dz, dDE/dpower,

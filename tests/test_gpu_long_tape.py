@@ -1,5 +1,5 @@
-"""The reverse-mode gradient over the long tape (every step's record, loops up
-to 20 iterations) against the checkpointed tape (adjoint_ck 4: segments
+"""The reverse-mode gradient over the long tape (every step's record, loops of 6
+to 30 iterations) against the checkpointed tape (adjoint_ck 4: segments
 recomputed).  Both sweep the same records through the same operations: the
 outputs have the same bits.  And the batch product and its sums against the
 per-point gradients."""
@@ -56,7 +56,7 @@ def test_batch_product_matches_points(cg, n, iters):
     assert ((got - total).abs() <= (n + 64) * 2.0 ** -24 * size + 1e-30).all()
 
 
-@pytest.mark.parametrize("iters", [9, 10, 17, 18])
+@pytest.mark.parametrize("iters", [6, 9, 10, 17, 18, 30, 31])
 @pytest.mark.parametrize("n", [1, 127, 129, 700001])
 def test_tensor_memory_columns(cg, n, iters):
     """Where the columns per block change (9, 17 steps), at the edges of a block
