@@ -117,7 +117,7 @@ __device__ __forceinline__ void warp_pool(const WarpWalk& w, uint64_t n, int wai
     const bool alike = wait == 32;
     uint32_t probe = max(max_steps / 5, 1u);
     bool have = false, busy = false;
-    while (wait < 32 || next > 0) {
+    while (!alike) {
         const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !busy);
         const uint32_t done = __ballot_sync(0xFFFFFFFFu, have && !busy);
         // Enough lanes wait for new points or, when there are none, with results.
@@ -143,7 +143,7 @@ __device__ __forceinline__ void warp_pool(const WarpWalk& w, uint64_t n, int wai
             if (!__any_sync(0xFFFFFFFFu, busy)) break;
         }
         if (busy) busy = task.step();
-        if (--probe == 0 && next == 32) wait = 32;
+        if (--probe == 0) wait = next == 32 ? 32 : wait;
     }
     // A grid's rows and a stride near a multiple of them would leave each warp
     // one part of the shape: the warps change places from group to group.
