@@ -71,7 +71,7 @@ __host__ ShapeDev make_shape_dev(const cg_shape& s) {
     d.rotated = s.rot[0] != 0.0f || s.rot[1] != 0.0f || s.rot[2] != 0.0f;
     d.m2_max = largest_square(s.bailout);
     d.m2_wide = std::isnan(d.m2_max) ? NAN : 0x1p40f;
-    d.p8_m2_max = s.max_iters >= 1 && s.bailout <= 16.0f ? d.m2_max : NAN;
+    d.p8_m2_max = s.max_iters >= 1 && s.bailout >= 0x1p-20f && s.bailout <= 16.0f ? d.m2_max : NAN;
     return d;
 }
 

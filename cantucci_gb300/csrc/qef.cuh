@@ -80,7 +80,8 @@ __device__ __forceinline__ bool p8_gradient_loop(uint32_t max_iters, float bailo
             out = m2.v > m2_max;
             if (!out && !(m2.v <= m2_max && rxy2.v >= kP8MinRxy2)) return false;
         }
-        r = NORMAL && !out ? d3sqrt<true>(m2) : d3sqrt<false>(m2);
+        // (the squares that escape have the short root's bits up to 2^40)
+        r = NORMAL && m2.v <= 0x1p40f ? d3sqrt<true>(m2) : d3sqrt<false>(m2);
         if (NORMAL ? out : r.v > bailout) break;
         // f32::powi(r, 7) = (r * r^2) * r^4, times P, times dr, plus 1
         const D3 r2 = d3mul(r, r), r4 = d3mul(r2, r2), r7 = d3mul(d3mul(r, r2), r4);

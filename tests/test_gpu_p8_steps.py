@@ -50,3 +50,14 @@ def test_shortened_step_same_bits(cg, name, iters, bailout):
            (0.1, 0.2, -np.inf), (1e-30, 0.2, 0.3), (0.7, 0.0, -0.0)]
     d = s.batch_min_distance_from(np.array(pts, np.float32))
     assert d.shape == (7,)  # every special point ends
+
+
+@pytest.mark.parametrize("bailout", [1e-6, 9e-7, 1e-15, 1e-21])
+@pytest.mark.parametrize("name", ["cube", "origin", "origin_tiny", "yz_denormal"])
+def test_tiny_bailouts_same_bits(cg, name, bailout):
+    """Squares that escape a bailout about 2^-20 and below it: the last root is
+    the shortened one only down to there."""
+    s = cg.Mandelbulb(8, 15, bailout)
+    ref = grid(cg, 3, s, SPANS[name], 32)
+    for variant in (1, 2):
+        assert np.array_equal(grid(cg, variant, s, SPANS[name], 32), ref), variant
