@@ -14,6 +14,7 @@
 #include "common.cuh"
 #include "de.cuh"
 #include "point_io.cuh"
+#include "pool_share.cuh"
 
 namespace cg {
 
@@ -89,10 +90,8 @@ __device__ __forceinline__ bool points_side_by_side(const float* __restrict__ pt
     return points_side_by_side(pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]);
 }
 
-// Runs `task` over this warp's points, groups of 32 consecutive ones from
-// w.first (< n) on, w.stride apart (each warp's share then spans the whole
-// batch, so that dense parts of it do not fall to a few warps).  Call from all
-// 32 lanes.
+// Runs `task` over this warp's share of the n points (pool_share.cuh; w.first <
+// n).  Call from all 32 lanes.
 //   task.start(i)   begin point i            task.step()  one step, false at the end
 //   task.finish(i)  write point i's result   task.steps() the steps of the point
 //   task.whole(i)   all of point i
@@ -108,11 +107,8 @@ template <class Task>
 __device__ __forceinline__ void warp_pool(const WarpWalk& w, uint64_t n, int wait,
                                           uint32_t max_steps, Task& task) {
     const uint32_t below = (1u << (threadIdx.x & 31)) - 1u;
-    // Point k of the warp's share is first + (k / 32) stride + k % 32.
-    const uint64_t groups = (n - w.first + w.stride - 1) / w.stride;
-    const uint64_t last = n - (w.first + (groups - 1) * w.stride);
-    const uint64_t count = (groups - 1) * 32 + (last < 32 ? last : 32);
-    uint64_t next = 0, mine = 0;
+    PoolShare share(w.first, w.stride, n);
+    uint64_t mine = 0;
     uint32_t ended = 0, steps = 0;
     const bool alike = wait == 32;
     uint32_t probe = max(max_steps / 5, 1u);
@@ -121,7 +117,7 @@ __device__ __forceinline__ void warp_pool(const WarpWalk& w, uint64_t n, int wai
         const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !busy);
         const uint32_t done = __ballot_sync(0xFFFFFFFFu, have && !busy);
         // Enough lanes wait for new points or, when there are none, with results.
-        const uint32_t waiting = next < count ? idle : done;
+        const uint32_t waiting = share.next < share.end ? idle : done;
         if (__popc(waiting) >= wait || idle == 0xFFFFFFFFu) {
             if (have && !busy) task.finish(mine);
             if (wait == 32) break;  // every lane has ended
@@ -134,26 +130,19 @@ __device__ __forceinline__ void warp_pool(const WarpWalk& w, uint64_t n, int wai
                 continue;
             }
             if (!busy) {
-                const uint64_t k = next + __popc(idle & below);
-                have = busy = k < count;
-                mine = w.first + (k >> 5) * w.stride + (k & 31);
+                mine = share.index(__popc(idle & below));
+                have = busy = mine < n;
                 if (have) task.start(mine);
             }
-            next += __popc(idle);
+            share.advance(__popc(idle));
             if (!__any_sync(0xFFFFFFFFu, busy)) break;
         }
         if (busy) busy = task.step();
-        if (--probe == 0) wait = next == 32 ? 32 : wait;
+        if (--probe == 0) wait = share.next == 32 ? 32 : wait;
     }
-    // A grid's rows and a stride near a multiple of them would leave each warp
-    // one part of the shape: the warps change places from group to group.
-    const uint64_t turn = alike ? (w.stride * 618 / 1000) & ~31ull : 0;
-    const uint64_t end = alike ? (n + w.stride - 1) / w.stride * 32 : count;
-    for (uint64_t first = w.first; next < end; next += 32) {
-        const uint64_t k = next + (threadIdx.x & 31), i = first + (k >> 5) * w.stride + (k & 31);
+    for (; share.next < share.end; share.advance(32)) {
+        const uint64_t i = share.index(threadIdx.x & 31);
         if (i < n) task.whole(i);
-        first += turn;
-        if (first >= w.stride) first -= w.stride;
     }
 }
 
