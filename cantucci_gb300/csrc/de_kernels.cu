@@ -48,6 +48,12 @@ struct PointTask {
 template <int M>
 constexpr int kPointFlush = M == MODE_P8 ? 12 : 8;
 
+// Blocks to an SM (pool_grid): 2 M uniform points, polar power 8, 168 us with 8,
+// 174 with 10, on the surface 272 and 274, but 1.7 M on it 238 and 229, 5 M 692
+// and 653; Mandelbulb<8>, 2 M uniform 76 and 80, 5 M 168 and 164.
+template <int M>
+constexpr uint32_t kPointBlocks = M == MODE_P8 ? 8 : 10;
+
 template <int M, int MU>
 __global__ void __launch_bounds__(128) k_de_points_pool(ShapeDev s, const float* __restrict__ pts,
                                                         uint64_t n, float* __restrict__ out) {
@@ -341,7 +347,7 @@ cg_status launch_grid_work(const ShapeDev& s, const GridDev& g, unsigned long lo
 template <int M, int MU = M>
 static bool launch_points_pool(const ShapeDev& s, const float* pts, uint64_t n, float* out,
                                cudaStream_t st) {
-    const unsigned G = pool_grid(k_de_points_pool<M, MU>, n);
+    const unsigned G = pool_grid(kPointBlocks<M>, n);
     if (G) k_de_points_pool<M, MU><<<G, 128, 0, st>>>(s, pts, n, out);
     return G != 0;
 }
@@ -349,11 +355,11 @@ static bool launch_points_pool(const ShapeDev& s, const float* pts, uint64_t n, 
 // True if the batch is large enough for a pool kernel (and was launched).  The
 // exact estimators only: a step of the fast ones is too short for it (9 M points
 // on the surface 4 to 8 % slower, 3 M points anywhere no faster).
-// In us, the plain kernel -> the pool: polar power 8,
-// 3 M uniform points 396 -> 236, 16 M 2082 -> 1080; 3 M on the surface 396 ->
-// 403, 16 M 2082 -> 2050; 9 M of a grid 510 -> 515; Mandelbulb<8>, 3 M uniform
-// 136 -> 109, on the surface 136 -> 126, a grid 74 -> 60; 1.7 M polar uniform
-// 225 -> 155, on the surface 225 -> 237.
+// In us, the plain kernel -> the pool: polar power 8, 3 M uniform points 383 ->
+// 235, 16 M 2008 -> 1061; 3 M on the surface 383 -> 399, 16 M 2008 -> 2014; 9 M
+// of a grid 496 -> 506; Mandelbulb<8>, 3 M uniform 115 -> 104, on the surface
+// 117 -> 123, a grid 61 -> 57; 1.7 M polar uniform 218 -> 152, on the surface
+// 217 -> 229.
 static bool launch_points_pool_mode(const ShapeDev& s, const float* pts, uint64_t n, float* out,
                                     uint32_t numerics, cudaStream_t st) {
     if (s.max_iters < 1) return false;

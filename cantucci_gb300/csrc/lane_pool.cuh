@@ -9,6 +9,7 @@
 // the range's next points together.
 #pragma once
 
+#include <algorithm>
 #include <cstdint>
 
 #include "common.cuh"
@@ -147,26 +148,16 @@ __device__ __forceinline__ void warp_pool(const WarpWalk& w, uint64_t n, int wai
 }
 
 // The blocks (of 128 threads) of a pool kernel over n points: 16 points to a
-// lane, between two and eight times the blocks that fit on the GPU at once
-// (blocks then end at different times and the SMs stay full: 209 against 253 us
-// for 3 M points of a grid at two, 868 against 805 for 16 M at five).  0 with
-// fewer than 8 points to a lane of the blocks that fit, where a pool gains less
-// than its uneven end costs (1 M points: uniform 135 -> 101 us, but on the
-// surface 135 -> 147 and of a grid 80 -> 92).
-template <class Kernel>
-unsigned pool_grid(Kernel kernel, uint64_t n) {
-    static int per_sm = 0;
-    if (!per_sm) {
-        int b = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, 128, 0) != cudaSuccess ||
-            b < 1)
-            b = 1;
-        per_sm = b;
-    }
-    const uint64_t lanes = (uint64_t)sm_count() * per_sm * 128;
-    if (n < 8 * lanes) return 0;
-    const uint64_t resident = lanes / 128, even = n / (16 * 128);
-    return (unsigned)std::min(std::max(even, 2 * resident), 8 * resident);
+// lane, between two and eight times `per_sm` to an SM (about what fits on it:
+// blocks then end at different times and the SMs stay full; 3 M points of a grid
+// take 193 us at two times ten, 205 at once).  0 with fewer than 8 points to a
+// lane of `per_sm` blocks, where a pool gains less than its uneven end costs (1.1
+// M points: uniform 145 -> 115 us, but on the surface 145 -> 154 and of a grid
+// 80 -> 88).  A function of n and the estimator alone.
+inline unsigned pool_grid(uint32_t per_sm, uint64_t n) {
+    const uint64_t resident = (uint64_t)sm_count() * per_sm;
+    if (n < 8 * 128 * resident) return 0;
+    return (unsigned)std::min(std::max(n / (16 * 128), 2 * resident), 8 * resident);
 }
 
 }  // namespace cg
