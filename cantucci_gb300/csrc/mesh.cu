@@ -770,9 +770,10 @@ static cg_status launch_cells(const MeshDims& d, const MeshWork& w, cudaStream_t
     }
     if (d.res <= kClusterRowsMaxRes) {
         const uint32_t words = rows << d.wshift;
-        static const cudaError_t cluster16 = cudaFuncSetAttribute(
-            k_rows_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        CG_CUDA(cluster16);
+        // (The attribute is the function's on the current device: set at every
+        // launch, since a process may mesh on several.  Graph replays skip it.)
+        CG_CUDA(cudaFuncSetAttribute(k_rows_cluster,
+                                     cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         const unsigned B = ((words + kRowsCluster - 1) / kRowsCluster + 31) & ~31u;
         k_rows_cluster<<<kRowsCluster, B, 0, st>>>(w.sgn, d, w.cellbits, w.wordoff, w.rowoff,
                                                    w.quadoff, w.cellidx, w.counters);
