@@ -33,15 +33,18 @@ def _shape(power: float, rot, max_iters: int, bailout: float) -> _ffi.CgShape:
     return s
 
 
-def split_params(params, power_device, rot_device):
+def split_params(params, power_device, rot_device, need_power=True, need_rot=True):
     """(d/dpower, d/drotation) of a 4-vector of parameter gradients on the
-    parameters' devices, in one transfer where they share one."""
+    parameters' devices, in one transfer where they share one; None, and no
+    transfer, for one that is not needed (a transfer to the host waits for the
+    GPU and cannot be captured)."""
     def move(t, device):
         return t if device is None else t.to(device)
 
-    if power_device == rot_device:
+    if need_power and need_rot and power_device == rot_device:
         params = move(params, power_device)
-    return move(params[0], power_device), move(params[1:4], rot_device)
+    return (move(params[0], power_device) if need_power else None,
+            move(params[1:4], rot_device) if need_rot else None)
 
 
 def _make_function():
@@ -76,9 +79,8 @@ def _make_function():
                                         C.c_void_p(gp.data_ptr()) if gp is not None else None,
                                         C.c_void_p(params.data_ptr()),
                                         C.c_void_p(stream.cuda_stream)))
-            gpow, grot = split_params(params, *ctx.param_devices)
-            return (gp, gpow if ctx.needs_input_grad[1] else None,
-                    grot if ctx.needs_input_grad[2] else None, None, None)
+            return (gp, *split_params(params, *ctx.param_devices, *ctx.needs_input_grad[1:3]),
+                    None, None)
 
     return MandelbulbDE
 
