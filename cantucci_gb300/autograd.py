@@ -33,6 +33,13 @@ def _shape(power: float, rot, max_iters: int, bailout: float) -> _ffi.CgShape:
     return s
 
 
+def angles(rot):
+    """The angles of a rotation tensor on the host, in one transfer: one scalar
+    per entry of the first dimension."""
+    rot = rot.detach()
+    return rot.tolist() if rot.dim() == 1 else [float(v) for v in rot.cpu()]
+
+
 def split_params(params, power_device, rot_device, need_power=True, need_rot=True):
     """(d/dpower, d/drotation) of a 4-vector of parameter gradients on the
     parameters' devices, in one transfer where they share one; None, and no
@@ -54,7 +61,7 @@ def _make_function():
         @staticmethod
         def forward(ctx, points, power, rot, max_iters, bailout):
             pts = points.detach().contiguous().float()
-            shape = _shape(float(power), rot.detach().reshape(-1).tolist(), max_iters, bailout)
+            shape = _shape(float(power), angles(rot), max_iters, bailout)
             out = torch.empty(pts.shape[0], dtype=torch.float32, device=pts.device)
             stream = torch.cuda.current_stream(pts.device)
             check(load().cg_min_distance_from(C.byref(shape), C.c_void_p(pts.data_ptr()),

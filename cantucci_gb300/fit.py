@@ -30,7 +30,7 @@ import math
 
 from . import _ffi
 from ._ffi import check, load
-from .autograd import split_params
+from .autograd import angles, split_params
 
 
 def _torch():
@@ -88,7 +88,7 @@ def _make_render_fn():
         @staticmethod
         def forward(ctx, power, rot, cam, max_steps, eps_scale, max_iters, bailout, fast, cap):
             p = float(power)
-            r = rot.detach().reshape(-1).tolist()
+            r = angles(rot)
             depth = render(p, r, cam, max_steps, eps_scale, max_iters, bailout, fast=fast)
             ctx.save_for_backward(depth)
             ctx.shape = _shape(p, r, max_iters, bailout)
@@ -180,7 +180,7 @@ def _make_surface_fn():
         def forward(ctx, power, rot, points, max_iters, bailout, cap):
             pts = points.contiguous().float()
             out = torch.empty(5, dtype=torch.float32, device=pts.device)
-            shape = _shape(float(power), rot.detach().reshape(-1).tolist(), max_iters, bailout)
+            shape = _shape(float(power), angles(rot), max_iters, bailout)
             check(load().cg_surface_l1(
                 C.byref(shape), C.c_void_p(pts.data_ptr()), pts.shape[0], max(float(cap), 0.0),
                 C.c_void_p(out.data_ptr()),
