@@ -1,8 +1,9 @@
 """The distance estimator as a torch.autograd.Function.
 
 forward:  cg_min_distance_from (the polar-form estimator, f32).
-backward: cg_de_backward -- the hand-written adjoint kernel, which recomputes
-          the iterates from checkpoints instead of saving them -- giving
+backward: cg_de_backward -- the hand-written adjoint kernel, which walks the loop
+          again and keeps every step's record on chip (6 to 30 steps) or
+          checkpoints of it; nothing but the points is saved -- giving
           dL/dpoints and dL/d(power, euler angles).
 
     power = torch.tensor(8.0, requires_grad=True)
@@ -109,7 +110,8 @@ def de_grad(points, power: float, rot=(0.0, 0.0, 0.0), max_iters: int = 15,
             fast: bool = False):
     """(n, 8) CUDA tensor: DE, dDE/dp (3), dDE/dpower, dDE/d(euler) (3).
 
-    mode "adjoint": reverse mode with checkpoint recompute (cg_de_grad).
+    mode "adjoint": reverse mode (cg_de_grad), every step's record on chip for 6 to
+    30 iterations, else segments recomputed from checkpoints.
     mode "tangent": forward mode, one pass (cg_de_grad_tangent); with
     with_power=False it skips the power direction (column 4 is 0), which is
     all a normal needs; fast=True iterates with the fast polar estimator's

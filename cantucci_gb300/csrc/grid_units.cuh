@@ -20,7 +20,6 @@ namespace cg {
 constexpr uint32_t kUnitMinRes = 32;
 
 // shift = log2 res.
-__host__ __device__ constexpr uint32_t core_bricks(uint32_t shift) { return 1u << (3 * shift - 5); }
 __host__ __device__ constexpr uint32_t core_units(uint32_t shift) { return 1u << (3 * shift - 8); }
 __host__ __device__ constexpr uint32_t face_row_items(uint32_t shift) {
     return ((2u << shift) + 1u) << (shift - 5);

@@ -550,7 +550,15 @@ cg_status cg_fd_grad(const cg_shape* shape, const float* points, uint64_t n, flo
  * "mesh_graphs" (1 default, or 0): meshes up to resolution 128 (other than
  * dual contouring) replay a CUDA graph the mesher captured for that
  * resolution, shape and option set, the span going in as a parameter block.
- * None of these changes an output bit.  "batch_block", "batch_chunk",
+ * "adjoint_ck" (5 default, 4 or 8): the checkpoint interval of cg_de_grad; 4 and 8
+ * also take loops of 6 to 30 steps off the long tape.
+ * None of these changes an output bit.  "adjoint_recompute" (0 default, or 1):
+ * cg_de_grad and cg_surface_l1 sweep checkpointed segments that are formed again
+ * in the fast polar arithmetic (the DE exact, the gradients not; autograd.py's
+ * and cg_de_backward's are exact either way).  Above 30 steps it saves the exact
+ * recompute; up to 30, where the default recomputes nothing, it is the slower one
+ * (1 M points of 15 steps, 283 against 215 us) and is best left at 0.
+ * "batch_block", "batch_chunk",
  * "batch_brick_min_res", "batch_place_block": the cg_batch_tuning that
  * batches created afterwards start with (defaults 256, 4, 8, 128). */
 cg_status cg_set_option(const char* name, int64_t value);
