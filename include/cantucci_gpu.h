@@ -555,9 +555,9 @@ cg_status cg_fd_grad(const cg_shape* shape, const float* points, uint64_t n, flo
  * None of these changes an output bit.  "adjoint_recompute" (0 default, or 1):
  * cg_de_grad and cg_surface_l1 sweep checkpointed segments that are formed again
  * in the fast polar arithmetic (the DE exact, the gradients not; autograd.py's
- * and cg_de_backward's are exact either way).  Above 30 steps it saves the exact
- * recompute; up to 30, where the default recomputes nothing, it is the slower one
- * (1 M points of 15 steps, 283 against 215 us) and is best left at 0.
+ * and cg_de_backward's are exact either way).  Worth it above 30 steps, where it
+ * saves the exact recompute (1 M points of 31 steps, 875 -> 652 us); from 6 to 30 the
+ * default recomputes nothing and is the faster one (15 steps, 219 against 283).
  * "batch_block", "batch_chunk",
  * "batch_brick_min_res", "batch_place_block": the cg_batch_tuning that
  * batches created afterwards start with (defaults 256, 4, 8, 128). */
